@@ -153,6 +153,7 @@ int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler) {
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     if (scheduler != 0 && scheduler != 1) return ctx->fail(TS_E_ARG, "scheduler must be 0 (lockstep) or 1 (flow)");
     ctx->scheduler = scheduler;
+    ctx->chosen_f64 = ctx->chosen_f32 = true;
     ctx->drop_graph();
     return TS_OK;
 }
@@ -166,6 +167,7 @@ int ts_engine_set_tile(ts_ctx* ctx, int32_t precision, int32_t shape_id) {
     if (precision == TS_PRECISION_F64) ctx->tile_f64 = shape_id;
     else if (precision == TS_PRECISION_F32) ctx->tile_f32 = shape_id;
     else return ctx->fail(TS_E_ARG, "precision must be 64 or 32");
+    (precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32) = true;
     return TS_OK;
 }
 

@@ -156,12 +156,16 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
     double best_ms = INFINITY;
     const int keep64 = ctx->tile_f64, keep32 = ctx->tile_f32, keep_sched = ctx->scheduler;
     const bool keep_graph = ctx->use_graph;
+    const bool keep_c64 = ctx->chosen_f64, keep_c32 = ctx->chosen_f32;
     ctx->use_graph = false;
+    ctx->chosen_f64 = ctx->chosen_f32 = true;  // the shapes are what is timed
     auto restore = [&]() {
         ctx->tile_f64 = keep64;
         ctx->tile_f32 = keep32;
         ctx->scheduler = keep_sched;
         ctx->use_graph = keep_graph;
+        ctx->chosen_f64 = keep_c64;
+        ctx->chosen_f32 = keep_c32;
     };
     // Every (shape, scheduler) pair; entry 2·q + scheduler of ms_per_shape.
     for (size_t q = 0; q < shapes.size(); q++) {
@@ -190,8 +194,8 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
         }
     }
     restore();
-    if (precision == TS_PRECISION_F64) ctx->tile_f64 = best;
-    else ctx->tile_f32 = best;
+    (precision == TS_PRECISION_F64 ? ctx->tile_f64 : ctx->tile_f32) = best;
+    (precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32) = true;
     ctx->scheduler = best_sched;
     ctx->drop_graph();
     *best_tile = best;

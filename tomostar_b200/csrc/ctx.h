@@ -26,6 +26,8 @@ struct ts_ctx {
     int* cancel_dev = nullptr;
     int tile_f64 = 0, tile_f32 = 0;       // engine tile shape per precision
     int scheduler = 0;                    // engine scheduler: 0 lockstep diagonals, 1 flow (per field)
+    // The caller has chosen a tile shape or scheduler (ts_engine_set_tile, _set_scheduler, the autotuner).
+    bool chosen_f64 = false, chosen_f32 = false;
     double epoch_budget_ms = 0;           // flow epochs: fields pause at the first round end after this
     // The extended domain's 1-D background for the rays' outside time (ts_set_background): node count,
     // the nodes in the "rays.background" buffer (depths, Vp, Vs).

@@ -7,6 +7,7 @@
 
 #include "eik_engine.h"
 #include "eik_engine_kernel.cuh"
+#include "eik_resident.h"
 
 namespace ts {
 namespace eik {
@@ -639,6 +640,10 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     job.pitch.clear();
     for (auto& L : layouts) job.pitch.push_back(L.pitch);
     job.xoff = layouts.empty() ? 0 : layouts[0].xoff;
+    // Small grids are solved in shared memory, a cluster per field, unless the caller has chosen a shape
+    // or a scheduler of the tiled engine, or wants the launch captured.
+    if (!(is_f64<Real>() ? ctx->chosen_f64 : ctx->chosen_f32) && !ctx->use_graph)
+        if (const int cluster = resident_cluster(ctx, job)) return resident_run<Real>(ctx, job, cluster, stats, ctx->stream);
     return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, job.tile, 0, stats, ctx->stream);
 }
 
