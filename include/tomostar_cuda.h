@@ -155,11 +155,13 @@ int ts_cuda_selftest(ts_ctx* ctx, int32_t precision, double* rel_err, char* msg,
 /* Engine tile shapes compiled into the library: writes up to cap (id, bx, by, bz) quadruples to
  * shapes and returns how many exist. No reference counterpart (the OpenCL kernel is untiled). */
 int32_t ts_engine_shapes(int32_t* shapes, int32_t cap);
-/* Selects the engine's tile shape for one precision on this context (the autotuner's knob). */
-/* Engine scheduler: 0 = all fields step through the tile diagonals together (one grid-wide barrier
- * per diagonal); 1 = flow: each field advances on its own through a shared tile queue (no barrier).
- * Both give the same fields. No reference counterpart. */
+/* Engine scheduler. Each field advances on its own through a shared tile queue; 1 also lets a server's
+ * epoch end on time (ts_serve_set_epoch_ms). Both give the same fields. No reference counterpart. */
 int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler);
+/* Selects the engine's tile shape for one precision on this context (the autotuner's knob): an id of
+ * ts_engine_shapes, or any id up to 10, which leaves the shape to each job. Without a call (and
+ * without ts_engine_set_scheduler) small grids are solved in the shared memory of one block cluster
+ * per field instead of in tiles. Every choice gives the same fields. */
 int ts_engine_set_tile(ts_ctx* ctx, int32_t precision, int32_t shape_id);
 
 /* Many fields on grids of uneven size in one engine launch (the reference batches only fields of one

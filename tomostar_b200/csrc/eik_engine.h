@@ -44,7 +44,7 @@ struct EngineJob {
     std::vector<EngineField> fields;
     double tol = 1e-7;
     double wake_rel = 0;     // 0: the reference's dirty rule (bitwise); TS_WAKE_REL for TS_MODE_FAST
-    int tile = 0;            // tile shape id
+    int tile = 0;            // tile shape id; engine_run sets the one it used
     // Set by the engine: the padded layout of each grid's fields.
     std::vector<int> pitch;
     int xoff = 0;
@@ -55,6 +55,10 @@ struct TileShapeInfo {
     int id, bx, by, bz;
 };
 const std::vector<TileShapeInfo>& tile_shapes();
+// Every tile has rows of 32 nodes; 16×8 rows (flat) or 16×16 (deep).
+constexpr int kTileX = 32, kTileFlat = 0, kTileDeep = 1, kTileLastId = 10;
+// Whether a caller may give this id (an id without a shape of its own leaves the choice to the job).
+bool tile_known(int id);
 
 // Layout of a field on a grid for a tile shape and precision: elements per padded row, x offset,
 // tiles, due-mask words per tile.

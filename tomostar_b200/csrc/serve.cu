@@ -69,7 +69,7 @@ struct ts_server {
     ts_ctx* ctx = nullptr;
     int precision = TS_PRECISION_F64;
     int mode = TS_MODE_FAST;
-    int tile = 2;
+    int tile = 0;
     int rounds_per_epoch = 1;
     size_t budget = 0;
     size_t in_use = 0, peak_use = 0;
@@ -408,9 +408,7 @@ int ts_serve_create(int32_t device, int32_t precision, int32_t mode, int32_t til
     if (precision != TS_PRECISION_F64 && precision != TS_PRECISION_F32) return TS_E_ARG;
     if (mode != TS_MODE_ENGINE && mode != TS_MODE_FAST) return TS_E_ARG;
     if (!(hbm_budget_bytes > 0)) return TS_E_ARG;
-    bool known = false;
-    for (const auto& t : ts::eik::tile_shapes()) known |= t.id == tile;
-    if (!known) return TS_E_ARG;
+    if (!ts::eik::tile_known(tile)) return TS_E_ARG;
     if (scheduler != 0 && scheduler != 1) return TS_E_ARG;
     ts_ctx* ctx = nullptr;
     int rc = ts_cuda_create(device, &ctx);
@@ -427,7 +425,7 @@ int ts_serve_create(int32_t device, int32_t precision, int32_t mode, int32_t til
     sv->ctx = ctx;
     sv->precision = precision;
     sv->mode = mode;
-    sv->tile = tile;
+    sv->tile = tile == ts::eik::kTileDeep ? tile : ts::eik::kTileFlat;  // one layout for the server's life
     sv->budget = size_t(hbm_budget_bytes);
     sv->rounds_per_epoch = rounds_per_epoch > 0 ? rounds_per_epoch : 1;
     sv->loop = std::thread(serve_loop, sv);
