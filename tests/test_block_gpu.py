@@ -60,3 +60,23 @@ def test_earlier_shape_ids_are_accepted(engine):
         assert np.array_equal(engine.solve(g, s, seeds), want)
     assert L.load().ts_engine_set_tile(engine.handle, 64, 11) == L.TS_E_ARG
     assert L.load().ts_engine_set_tile(engine.handle, 64, -1) == L.TS_E_ARG
+
+
+@pytest.mark.parametrize("layered", [False, True])
+def test_ties_equal_the_oracle(engine, layered):
+    """Constant and layered media on a square grid: candidates whose roots equal a neighbour's time to
+    the last bits, where the choice of the terms is decided by the formed roots."""
+    from oracle import oracle as O
+
+    g = regular_grid(34, 34, 18, 1.0)
+    s = np.full(g.count, 0.2)
+    if layered:
+        s.reshape(g.shape)[9:] = 0.125
+    seeds = [point_source(g, s, *map(float, km_to_geo(g, 16.0, 16.0, 1.0)), 8.0),
+             point_source(g, s, g.min_lon, g.min_lat, 0.0)]
+    for sid, *_ in L.engine_shapes():
+        shape(engine, sid)
+        got = engine.solve(g, s, seeds, mode=L.MODE_ENGINE, precision=64)
+        for f, (idx, t) in enumerate(seeds):
+            want = O.relax(O.Grid.of(g), s, idx, t)
+            assert np.array_equal(got[f], (want[0] if isinstance(want, tuple) else want).reshape(-1))

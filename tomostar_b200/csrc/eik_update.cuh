@@ -49,27 +49,29 @@ TS_DEVINL double ddiv3(double a) {
 }
 
 // One axis's term (SphericalEikonal.cs:381-395): the smaller neighbour, promoted to second order
-// when its partner beyond is finite and not larger. Produces (effective time, weight, neighbour
-// time); unused terms keep t = +inf and sort last.
+// when its partner beyond is finite and not larger (a partner not larger than a finite neighbour is
+// finite). Produces (effective time, weight, neighbour time) by selections alone, so that the lanes of a
+// warp stay together; an axis with no finite neighbour gives t = n = +inf, which sorts last, and does
+// not count as used.
 template <bool VARZ>
 TS_DEVINL void axis64(double minus, double plus, double minus2, double plus2, double w1, double w2, const double* zc,
                       bool second, double& te, double& we, double& tn, int& used) {
-    double first, t2;
-    bool minus_side = minus <= plus;
-    if (minus_side) { first = minus; t2 = minus2; }
-    else { first = plus; t2 = plus2; }
-    if (!(first <= 1.7976931348623157e308)) return;  // not finite (first is never NaN)
-    bool promote = second && (t2 <= 1.7976931348623157e308) && t2 <= first;
+    const bool minus_side = minus <= plus;
+    const double first = minus_side ? minus : plus, t2 = minus_side ? minus2 : plus2;
+    const bool finite = first <= 1.7976931348623157e308;  // first is never NaN
+    const bool promote = second && finite && t2 <= first;
     if (!VARZ) {
-        if (promote) { te = ddiv3(dsub(dmul(4.0, first), t2)); we = w2; }
-        else { te = first; we = w1; }
+        const double e = ddiv3(dsub(dmul(4.0, first), t2));
+        te = promote ? e : first;
+        we = promote ? w2 : w1;
     } else {
         const double* c = zc + (minus_side ? 0 : 8);
+        te = first;
+        we = c[0];
         if (promote) { te = ddiv(dsub(dmul(c[3], first), dmul(c[4], t2)), c[2]); we = c[1]; }
-        else { te = first; we = c[0]; }
     }
     tn = first;
-    used++;
+    used += finite ? 1 : 0;
 }
 
 // Stable sort of three (t, h, n) by t (SphericalEikonal.cs:246-254, 262-275).
@@ -101,17 +103,27 @@ TS_DEVINL Sums64 add_term(Sums64 q, double w, double t) {
     return q;
 }
 
-// The candidate of `terms` terms from their sums; false when the discriminant is negative or the root
-// falls below a neighbour it used.
-TS_DEVINL bool root_from(const Sums64& q, int terms, const double* n, double s, double& root) {
-    const double disc = dsub(dmul(q.swt, q.swt), dmul(q.sw, dsub(q.swt2, dmul(s, s))));
-    if (disc < 0.0) return false;
-    root = ddiv(dadd(q.swt, __dsqrt_rn(disc)), q.sw);
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-        if (r < terms && root < n[r]) return false;
-    return true;
+// Which of a node's candidates holds, without forming them. The candidate of k terms is refused when its
+// discriminant is negative or it falls below the largest neighbour n that it used, and the reference then
+// drops a term (SphericalEikonal.cs:364-378). With S = sqrt(disc), root = (swt + S) / sw is not below n
+// exactly when v = sw·n − swt does not exceed S: v <= 0 or v² <= disc. Rounding can only disagree with
+// the formed root where v and S differ by a few ulps of |swt| + |sw·n|; a margin of 1e-14 of that sum
+// (about 40 times their error) calls those cases unclear, and the caller forms the roots. So the
+// lanes of a warp that drop a term spend some 20 instructions on it and not a square root and a quotient
+// each: a lone warp's dependent updates take 710 cycles each where they took 815, and 920 against 1,640
+// when its lanes differ in the terms they keep.
+struct RootTest {
+    bool holds, falls;  // neither: unclear
+};
+
+TS_DEVINL RootTest test_root(const Sums64& q, double disc, double n) {
+    const double pn = dmul(q.sw, n), v = dsub(pn, q.swt), m = dmul(1e-14, dadd(fabs(q.swt), fabs(pn)));
+    const double hi = dadd(v, m), lo = dsub(v, m);
+    const bool real = !(disc < 0.0);
+    return {real && (hi <= 0.0 || dmul(hi, hi) <= disc), !real || (lo > 0.0 && dmul(lo, lo) > disc)};
 }
+
+TS_DEVINL double disc_of(const Sums64& q, double s2) { return dsub(dmul(q.swt, q.swt), dmul(q.sw, dsub(q.swt2, s2))); }
 
 // RelaxNode (SphericalEikonal.cs:349-379): the candidate time of a node from its 12 neighbour
 // values (+inf off the grid). xm/xp = i∓1, xm2/xp2 = i∓2, likewise y and z; (w1, w2) are each
@@ -122,7 +134,7 @@ TS_DEVINL double update64(double s, double xm, double xp, double xm2, double xp2
                           double wy1, double wy2, double wz1, double wz2, const double* zc, bool second) {
     const double inf = dinf();
     if (!(s > 0.0)) return inf;
-    double t[3] = {inf, inf, inf}, w[3] = {1.0, 1.0, 1.0}, n[3] = {inf, inf, inf};
+    double t[3], w[3], n[3];
     int used = 0;
     axis64<false>(xm, xp, xm2, xp2, wx1, wx2, nullptr, second, t[0], w[0], n[0], used);
     axis64<false>(ym, yp, ym2, yp2, wy1, wy2, nullptr, second, t[1], w[1], n[1], used);
@@ -132,10 +144,36 @@ TS_DEVINL double update64(double s, double xm, double xp, double xm2, double xp2
     const Sums64 q1 = add_term(Sums64{0.0, 0.0, 0.0}, w[0], t[0]);
     const Sums64 q2 = add_term(q1, w[1], t[1]);
     const Sums64 q3 = add_term(q2, w[2], t[2]);
-    double root;
-    if (used >= 3 && root_from(q3, 3, n, s, root)) return root;
-    if (used >= 2 && root_from(q2, 2, n, s, root)) return root;
-    if (root_from(q1, 1, n, s, root)) return root;
+    const double s2 = dmul(s, s);
+    const double n2 = fmax(n[0], n[1]);  // the largest neighbour of two terms; of three: with n[2]
+    // The first candidate, from the most terms, that holds (the one of one term is formed and tested). The
+    // choice is made before any root, so the lanes share one square root and one quotient; a warp whose
+    // lanes all hold three terms skips the rest of it.
+    double sw = q3.sw, swt = q3.swt, disc = disc_of(q3, s2);
+    const RootTest r3 = test_root(q3, disc, fmax(n2, n[2]));
+    const bool k3 = used == 3 && !r3.falls;
+    bool k2 = false, clear = r3.holds;
+    if (__any_sync(__activemask(), !k3)) {
+        const double d2 = disc_of(q2, s2), d1 = disc_of(q1, s2);
+        const RootTest r2 = test_root(q2, d2, n2);
+        k2 = !k3 && used >= 2 && !r2.falls;
+        clear = k3 ? r3.holds : k2 ? r2.holds : true;
+        sw = k3 ? sw : k2 ? q2.sw : q1.sw;
+        swt = k3 ? swt : k2 ? q2.swt : q1.swt;
+        disc = k3 ? disc : k2 ? d2 : d1;
+    }
+    if (clear) {
+        const double root = ddiv(dadd(swt, __dsqrt_rn(disc < 0.0 ? 0.0 : disc)), sw);
+        return !(k3 || k2) && (disc < 0.0 || root < n[0]) ? inf : root;
+    }
+    // The reference's own order of trials (rare).
+    for (int k = used; k >= 1; k--) {
+        const Sums64 q = k == 3 ? q3 : k == 2 ? q2 : q1;
+        const double d = disc_of(q, s2);
+        if (d < 0.0) continue;
+        const double root = ddiv(dadd(q.swt, __dsqrt_rn(d)), q.sw);
+        if (!(root < (k == 1 ? n[0] : k == 2 ? n2 : fmax(n2, n[2])))) return root;
+    }
     return inf;
 }
 
@@ -153,6 +191,14 @@ TS_DEVINL float fmul(float a, float b) { return __fmul_rn(a, b); }
 TS_DEVINL float fadd(float a, float b) { return __fadd_rn(a, b); }
 TS_DEVINL float fsub(float a, float b) { return __fadd_rn(a, -b); }
 TS_DEVINL float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// a / 3 correctly rounded (see ddiv3): the same bits as the quotient for every finite float a >= 0
+// (compared over all of them), in three instructions.
+TS_DEVINL float fdiv3(float a) {
+    const float third = 0.333333343f;  // RN(1/3)
+    const float q0 = __fmul_rn(a, third);
+    return __fmaf_rn(__fmaf_rn(-3.0f, q0, a), third, q0);
+}
 
 // df_sub: (a.hi − b.hi) + (a.lo − b.lo).
 TS_DEVINL float psub(Pair a, Pair b) { return fadd(fsub(a.hi, b.hi), fsub(a.lo, b.lo)); }
@@ -191,7 +237,7 @@ TS_DEVINL void termp(const PickP& p, Pair r, float w1, float w2, const Pair* zc,
     const float of = psub(p.first, r);
     const bool promote = second && finite_r(p.t2.hi) && !pless(p.first, p.t2);
     if (!VARZ) {
-        if (promote) { te = fadd(of, fdiv(psub(p.first, p.t2), 3.0f)); we = w2; }
+        if (promote) { te = fadd(of, fdiv3(psub(p.first, p.t2))); we = w2; }
         else { te = of; we = w1; }
     } else {
         const Pair* c = zc + (p.minus_side ? 0 : 8);
