@@ -2,10 +2,10 @@
 // (Location/EventLocator.cs:59-104) for many events at once, as Relocation.Absolute runs it
 // (Location/Relocation.cs:76-91).
 //
-// Per round (at most three): the grid search (EventLocator.cs:107-163) as one thread per candidate
-// node, so that the reads of one table by a warp's consecutive candidates coalesce; each candidate's
-// residuals are put in order by a stable insertion sort for the weighted-median origin time
-// (:297-309) and every sum is taken in the reference's order, so the best node and its origin time
+// Per round (at most three): the grid search (EventLocator.cs:107-163), a warp per candidate node where
+// weight sums are exact (the quality classes), its weighted-median origin time (:297-309) found by
+// selection; otherwise, and above 128 picks, a thread per candidate with a stable insertion sort. Sums
+// that decide are taken in the reference's order, so the best node and its origin time
 // equal the sequential search's. Then Geiger's Levenberg-Marquardt iterations (:166-256) and the
 // outlier rule (:84-90) as one warp per event: lanes evaluate observations (trilinear time and
 // gradient on the float32 tables) and every lane forms the normal equations in observation order
@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.h"
@@ -185,122 +186,138 @@ __global__ void __launch_bounds__(kSearchThreads) search_kernel(const SearchTask
     block_best(m, cc, partial);
 }
 
-// Bitonic sort of 32*E (key, pick) pairs held E per lane (element j*32 + lane in slot j), ascending by
-// key then pick: a total order, so the result is the stable sort by key.
-template <int E>
-__device__ __forceinline__ void warp_bitonic(double (&key)[E], int (&q)[E], int lane) {
-    constexpr int N = 32 * E;
-#pragma unroll
-    for (int k = 2; k <= N; k <<= 1) {
-#pragma unroll
-        for (int d = k >> 1; d > 0; d >>= 1) {
-            if (d >= 32) {
-#pragma unroll
-                for (int j = 0; j < E; j++) {
-                    const int jp = j ^ (d >> 5);
-                    if (jp > j) {
-                        const bool up = (((j * 32 + lane) & k) == 0);
-                        const bool gt = key[j] > key[jp] || (key[j] == key[jp] && q[j] > q[jp]);
-                        if (gt == up) {
-                            const double tk = key[j];
-                            key[j] = key[jp];
-                            key[jp] = tk;
-                            const int tq = q[j];
-                            q[j] = q[jp];
-                            q[jp] = tq;
-                        }
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < E; j++) {
-                    const double ok = __shfl_xor_sync(kFull, key[j], d);
-                    const int oq = __shfl_xor_sync(kFull, q[j], d);
-                    const bool up = (((j * 32 + lane) & k) == 0);
-                    const bool lower = (lane & d) == 0;
-                    const bool gt = key[j] > ok || (key[j] == ok && q[j] > oq);
-                    if (lower ? (gt == up) : (gt != up)) {
-                        key[j] = ok;
-                        q[j] = oq;
-                    }
-                }
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);
     return v;
 }
 
-// GridSearch's Misfit at one node by one warp, for dyadic non-negative weights (sums of at most 128
-// of them are exact in any order): the weighted-median origin time exactly as the reference's, and
-// the misfit either as a tree sum (fast) or in pick order (exact, the reference's rounding).
+// One event's picks as a warp holds them, E per lane (pick j*32 + lane in slot j). The weights are
+// multiples of 2^-24 below 2^18 (checked on the host): as whole numbers of 2^-24 they have 42 bits, kept
+// as two halves of 21, so that sums over a warp are two whole-number reductions, exact in any order.
 template <int E>
-__device__ double warp_node_misfit(const ObsD* so, int n, int64_t idx, int lane, bool exact) {
-    double key[E], r0[E], w0[E];
-    int q[E];
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-        const int qq = j * 32 + lane;
-        r0[j] = dnan();
-        w0[j] = 0;
-        key[j] = dinf();
-        q[j] = 1024 + qq;  // padding sorts after every pick
-        if (qq < n) {
-            const float t = __ldg(so[qq].tb + idx);
-            w0[j] = so[qq].w;
-            q[j] = qq;
-            if (isfinite(t)) {
-                r0[j] = so[qq].sec - double(t) - so[qq].corr;
-                key[j] = r0[j];
-            }
-        }
-    }
-    warp_bitonic<E>(key, q, lane);
-    // Weights in sorted order (finite residuals only), their total and inclusive prefix sums.
-    double ws[E];
-    double total = 0;
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-        ws[j] = (key[j] < dinf()) ? so[q[j]].w : 0.0;
-        total += ws[j];
-    }
-    total = warp_sum(total);
-    const double half = total / 2;
-    const unsigned finite0 = __ballot_sync(kFull, key[0] < dinf());
-    double t0 = 0;
-    if (finite0 != 0) {
-        double carry = 0;
-        bool found = false;
-        double last = 0;
+struct WarpPicks {
+    const float* tb[E];  // null: no pick
+    double sec[E], corr[E], w[E];
+    unsigned wlo[E], whi[E];
+
+    __device__ __forceinline__ void load(const ObsD* o, int n, int lane) {
 #pragma unroll
         for (int j = 0; j < E; j++) {
-            double x = ws[j];
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const double y = __shfl_up_sync(kFull, x, d);
-                if (lane >= d) x += y;
-            }
-            const double acc = carry + x;
-            carry += __shfl_sync(kFull, x, 31);
-            const unsigned fin = __ballot_sync(kFull, key[j] < dinf());
-            if (fin) last = __shfl_sync(kFull, key[j], 31 - __clz(fin));
-            const unsigned hit = __ballot_sync(kFull, key[j] < dinf() && acc >= half);
-            if (!found && hit) {
-                t0 = __shfl_sync(kFull, key[j], __ffs(hit) - 1);
-                found = true;
-            }
+            const int q = j * 32 + lane;
+            const ObsD v = q < n ? o[q] : ObsD{nullptr, 0, 0, 0};
+            tb[j] = v.tb;
+            sec[j] = v.sec;
+            corr[j] = v.corr;
+            w[j] = v.w;
+            const unsigned long long u = (unsigned long long)(v.w * 16777216.0);
+            wlo[j] = unsigned(u & 0x1fffffull);
+            whi[j] = unsigned(u >> 21);
         }
-        if (!found) t0 = last;
     }
+};
+
+// The sum over the warp of each lane's (hi, lo) half-weights, in units of 2^-24.
+__device__ __forceinline__ unsigned long long warp_weight(unsigned hi, unsigned lo) {
+    return ((unsigned long long)__reduce_add_sync(kFull, hi) << 21) + __reduce_add_sync(kFull, lo);
+}
+
+// The weighted median of EventLocator.cs:297-309 over the finite residuals (r < +inf): in the order of
+// (residual, pick) the first whose cumulative weight reaches half the total; 0 when there is none. The
+// order is not formed: a pivot splits what is left (the weight before it is one masked sum), the part
+// that cannot hold the median goes, some six times for 48 picks where a sort of 64 takes 21 exchange
+// stages: 400 events of 48 picks on 161×161×81 tables take 18 ms where sorting 128 took 91. `hint`: a pick to try first, and
+// the median's pick on return.
+template <int E>
+__device__ __forceinline__ double warp_median(const WarpPicks<E>& o, const double (&r)[E], int lane, int& hint) {
+    bool left[E];
+    unsigned lo = 0, hi = 0;
+#pragma unroll
+    for (int j = 0; j < E; j++) {
+        left[j] = r[j] < dinf();
+        lo += left[j] ? o.wlo[j] : 0u;
+        hi += left[j] ? o.whi[j] : 0u;
+    }
+    const unsigned long long total = warp_weight(hi, lo);
+    double median = 0;
+    int at = -1;
+    int pivot = hint;
+    {
+        bool on = false;
+#pragma unroll
+        for (int j = 0; j < E; j++) on = on || (left[j] && j * 32 + lane == pivot);
+        if (!__any_sync(kFull, on)) pivot = -1;
+    }
+    bool below[E];
+    for (;;) {
+        if (pivot < 0) {  // the first pick left
+#pragma unroll
+            for (int j = E - 1; j >= 0; j--) {
+                const unsigned m = __ballot_sync(kFull, left[j]);
+                if (m) pivot = j * 32 + __ffs(m) - 1;
+            }
+            if (pivot < 0) break;
+        }
+        double key = r[0];
+        unsigned plo = o.wlo[0], phi = o.whi[0];
+#pragma unroll
+        for (int j = 1; j < E; j++)
+            if ((pivot >> 5) == j) {
+                key = r[j];
+                plo = o.wlo[j];
+                phi = o.whi[j];
+            }
+        key = __shfl_sync(kFull, key, pivot & 31);
+        plo = __shfl_sync(kFull, plo, pivot & 31);
+        phi = __shfl_sync(kFull, phi, pivot & 31);
+        lo = hi = 0;
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+            below[j] = r[j] < key || (r[j] == key && j * 32 + lane < pivot);  // a NaN or +inf residual is not
+            lo += below[j] ? o.wlo[j] : 0u;
+            hi += below[j] ? o.whi[j] : 0u;
+        }
+        const unsigned long long before = warp_weight(hi, lo);
+        const bool reached = 2 * (before + ((unsigned long long)phi << 21) + plo) >= total;
+        if (reached) {
+            median = key;
+            at = pivot;
+            if (2 * before < total) break;  // and not by the one before
+        }
+#pragma unroll
+        for (int j = 0; j < E; j++) left[j] = left[j] && j * 32 + lane != pivot && below[j] == reached;
+        pivot = -1;
+    }
+    hint = at;
+    return median;
+}
+
+// GridSearch's residuals (EventLocator.cs:111-116) from the picks' table times at one node: NaN where
+// a table holds no time.
+template <int E>
+__device__ __forceinline__ void warp_residuals(const WarpPicks<E>& o, const float (&t)[E], double (&r)[E]) {
+#pragma unroll
+    for (int j = 0; j < E; j++) r[j] = o.tb[j] && isfinite(t[j]) ? o.sec[j] - double(t[j]) - o.corr[j] : dnan();
+}
+
+template <int E>
+__device__ __forceinline__ void warp_times(const WarpPicks<E>& o, int64_t idx, float (&t)[E]) {
+#pragma unroll
+    for (int j = 0; j < E; j++) t[j] = o.tb[j] ? __ldg(o.tb[j] + idx) : 0.f;
+}
+
+// GridSearch's Misfit at one node by one warp, from its residuals: the weighted-median origin time as the
+// reference's, and the misfit either as a tree sum (fast) or in pick order (exact, the reference's
+// rounding).
+template <int E>
+__device__ __forceinline__ double warp_misfit(const WarpPicks<E>& o, const double (&r)[E], int n, int lane, bool exact,
+                                              int& hint) {
+    const double t0 = warp_median<E>(o, r, lane, hint);
     double term[E];
     double m = 0;
 #pragma unroll
     for (int j = 0; j < E; j++) {
-        term[j] = (j * 32 + lane < n) ? (isnan(r0[j]) ? 10 * w0[j] : w0[j] * fabs(r0[j] - t0)) : 0.0;
+        term[j] = o.tb[j] ? (isnan(r[j]) ? 10 * o.w[j] : o.w[j] * fabs(r[j] - t0)) : 0.0;
         m += term[j];
     }
     if (!exact) return warp_sum(m);
@@ -320,26 +337,46 @@ constexpr int kWarpCands = 8;
 constexpr int kBlockCands = kWarpCands * (kSearchThreads / 32);
 
 template <int E>
-__global__ void __launch_bounds__(kSearchThreads, 4) search_warp_kernel(const SearchTask* __restrict__ tasks,
-                                                                     int n_tasks, const int* __restrict__ off,
-                                                                     const EvState* __restrict__ st,
-                                                                     const ObsD* __restrict__ olist, int nx, int ny,
-                                                                     Partial* __restrict__ partial) {
-    __shared__ ObsD so[32 * E];
+__global__ void __launch_bounds__(kSearchThreads, E <= 2 ? 4 : 3)
+    search_warp_kernel(const SearchTask* __restrict__ tasks, int n_tasks, const int* __restrict__ off,
+                       const EvState* __restrict__ st, const ObsD* __restrict__ olist, int nx, int ny,
+                       Partial* __restrict__ partial) {
     __shared__ double fm[kBlockCands];
     __shared__ double fmin_s;
     const SearchTask t = tasks[task_of_block(tasks, n_tasks)];
     const int n = st[t.event].nused;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) so[q] = olist[off[t.event] + q];
-    __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WarpPicks<E> picks;
+    picks.load(olist + off[t.event], n, lane);
     const int cb = (int(blockIdx.x) - t.block0) * kBlockCands;
-    for (int k = 0; k < kWarpCands; k++) {
-        const int slot = warp * kWarpCands + k;
-        const int c = cb + slot;
-        double m = dinf();
-        if (c < t.count) m = warp_node_misfit<E>(so, n, candidate_node(t, c, nx, ny), lane, false);
-        if (lane == 0) fm[slot] = m;
+    const int c0 = cb + warp * kWarpCands;
+    int hint = -1;
+    {
+        // The warp's candidates are consecutive: their nodes by steps of the box, the next one's times
+        // loaded while this one's median is found.
+        int ii = c0 % t.ci, jj = (c0 / t.ci) % t.cj, kk = c0 / (t.ci * t.cj);
+        auto node = [&] {
+            return (int64_t(t.k0 + kk * t.stride) * ny + t.j0 + jj * t.stride) * nx + t.i0 + ii * t.stride;
+        };
+        float next[E];
+        if (c0 < t.count) warp_times<E>(picks, node(), next);
+        for (int k = 0; k < kWarpCands; k++) {
+            double m = dinf();
+            if (c0 + k < t.count) {
+                double r[E];
+                warp_residuals<E>(picks, next, r);
+                if (++ii == t.ci) {
+                    ii = 0;
+                    if (++jj == t.cj) {
+                        jj = 0;
+                        kk++;
+                    }
+                }
+                if (k + 1 < kWarpCands && c0 + k + 1 < t.count) warp_times<E>(picks, node(), next);
+                m = warp_misfit<E>(picks, r, n, lane, false, hint);
+            }
+            if (lane == 0) fm[warp * kWarpCands + k] = m;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -355,7 +392,11 @@ __global__ void __launch_bounds__(kSearchThreads, 4) search_warp_kernel(const Se
         const int slot = warp * kWarpCands + k;
         const int c = cb + slot;
         if (c >= t.count || !(fm[slot] <= band)) continue;
-        const double m = warp_node_misfit<E>(so, n, candidate_node(t, c, nx, ny), lane, true);
+        float times[E];
+        double r[E];
+        warp_times<E>(picks, candidate_node(t, c, nx, ny), times);
+        warp_residuals<E>(picks, times, r);
+        const double m = warp_misfit<E>(picks, r, n, lane, true, hint);
         if (m < best || bc == 0x7fffffff) {
             best = m;
             bc = c;
@@ -369,8 +410,28 @@ __global__ void __launch_bounds__(kSearchThreads, 4) search_warp_kernel(const Se
     block_best(lane == 0 ? best : dinf(), lane == 0 ? bc : 0x7fffffff, partial);
 }
 
-// The best candidate of each task over its blocks (first minimum in scan order; every misfit +inf
-// gives the first candidate, as Search returns Index(i0, j0, k0)), its node, origin time and place.
+// The best candidate of a task over its blocks: the first minimum in scan order; every misfit +inf gives
+// the first candidate, as Search returns Index(i0, j0, k0).
+struct Best {
+    double m;
+    int c;
+};
+
+// Writes the best node, its place and origin time to the event and to best_out.
+__device__ __forceinline__ void set_best(const RGrid& g, const SearchTask& t, int c, double t0, int fix_depth, EvState& s,
+                                         int* best_out) {
+    const int ii = t.i0 + (c % t.ci) * t.stride;
+    const int jj = t.j0 + ((c / t.ci) % t.cj) * t.stride;
+    const int kk = t.k0 + (c / (t.ci * t.cj)) * t.stride;
+    s.best = int((int64_t(kk) * g.ny + jj) * g.nx + ii);
+    s.lon = g.min_lon + ii * g.dlon;
+    s.lat = g.min_lat + jj * g.dlat;
+    s.dep = fix_depth ? s.sdep : g.min_dep + kk * g.ddep;
+    s.t0 = t0;
+    *best_out = s.best;
+}
+
+// One thread per task (the thread search's events).
 template <int NMAX>
 __global__ void pick_best(const RGrid g, const SearchTask* __restrict__ tasks, int n_tasks,
                           const Partial* __restrict__ partial, const int* __restrict__ off,
@@ -380,27 +441,50 @@ __global__ void pick_best(const RGrid g, const SearchTask* __restrict__ tasks, i
     if (k >= n_tasks) return;
     const SearchTask t = tasks[k];
     const int nb = (t.count + per_block - 1) / per_block;
-    double bm = partial[t.block0].m;
-    int bc = partial[t.block0].c;
-    for (int b = 1; b < nb; b++)
-        if (partial[t.block0 + b].m < bm) {
-            bm = partial[t.block0 + b].m;
-            bc = partial[t.block0 + b].c;
-        }
-    if (!(bm < dinf())) bc = 0;
-    const int ii = t.i0 + (bc % t.ci) * t.stride;
-    const int jj = t.j0 + ((bc / t.ci) % t.cj) * t.stride;
-    const int kk = t.k0 + (bc / (t.ci * t.cj)) * t.stride;
-    const int64_t idx = (int64_t(kk) * g.ny + jj) * g.nx + ii;
+    Best b{partial[t.block0].m, partial[t.block0].c};
+    for (int q = 1; q < nb; q++)
+        if (partial[t.block0 + q].m < b.m) b = Best{partial[t.block0 + q].m, partial[t.block0 + q].c};
+    if (!(b.m < dinf())) b.c = 0;
     EvState& s = st[t.event];
     double t0;
-    node_misfit<NMAX>(olist + off[t.event], s.nused, idx, t0);
-    s.best = int(idx);
-    s.lon = g.min_lon + ii * g.dlon;
-    s.lat = g.min_lat + jj * g.dlat;
-    s.dep = fix_depth ? s.sdep : g.min_dep + kk * g.ddep;
-    s.t0 = t0;
-    best_out[k] = int(idx);
+    node_misfit<NMAX>(olist + off[t.event], s.nused, candidate_node(t, b.c, g.nx, g.ny), t0);
+    set_best(g, t, b.c, t0, fix_depth, s, &best_out[k]);
+}
+
+// One warp per task (the warp search's): the lanes share the scan over the blocks and the picks of the
+// origin time; a thread alone took longer over its sort than the search over its boxes.
+template <int E>
+__global__ void pick_best_warp(const RGrid g, const SearchTask* __restrict__ tasks, int n_tasks,
+                               const Partial* __restrict__ partial, const int* __restrict__ off,
+                               const ObsD* __restrict__ olist, EvState* __restrict__ st, int fix_depth, int per_block,
+                               int* __restrict__ best_out) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= n_tasks) return;  // the whole warp
+    const SearchTask t = tasks[k];
+    const int nb = (t.count + per_block - 1) / per_block;
+    // Blocks are in scan order and so are their candidates: the first minimum is the smallest (m, c).
+    Best b{dinf(), 0x7fffffff};
+    for (int q = lane; q < nb; q += 32) {
+        const Partial p = partial[t.block0 + q];
+        if (p.m < b.m) b = Best{p.m, p.c};
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const double m2 = __shfl_xor_sync(kFull, b.m, d);
+        const int c2 = __shfl_xor_sync(kFull, b.c, d);
+        if (better(m2, c2, b.m, b.c)) b = Best{m2, c2};
+    }
+    if (!(b.m < dinf())) b.c = 0;
+    EvState& s = st[t.event];
+    WarpPicks<E> picks;
+    picks.load(olist + off[t.event], s.nused, lane);
+    float times[E];
+    double r[E];
+    warp_times<E>(picks, candidate_node(t, b.c, g.nx, g.ny), times);
+    warp_residuals<E>(picks, times, r);
+    int hint = -1;
+    const double t0 = warp_median<E>(picks, r, lane, hint);
+    if (lane == 0) set_best(g, t, b.c, t0, fix_depth, s, &best_out[k]);
 }
 
 // Math.Max and Math.Clamp of .NET (NaN propagates; Max prefers +0 over -0).
@@ -742,7 +826,7 @@ namespace {
 
 constexpr int kMaxObs = 1024;  // observations per event (the search kernels' scratch)
 
-int obs_class(int n) { return n <= 32 ? 0 : n <= 128 ? 1 : 2; }
+int obs_class(int n) { return n <= 128 ? std::max(0, (n - 1) / 32) : 4; }
 
 // GeoMath.Azimuth (Geo/GeoMath.cs:98-107) and EventLocator.Gap (Location/EventLocator.cs:320-327).
 double azimuth_deg(double lon1, double lat1, double lon2, double lat2) {
@@ -798,14 +882,17 @@ int run_search(ts_ctx* ctx, const RGrid& rg, std::vector<SearchTask>& tasks, con
     TS_BUF(ctx, part_d, Partial, "loc.partial", std::max(1, blocks));
     TS_BUF(ctx, best_d, int, "loc.best", std::max(1, nt));
     TS_CUDA_TRY(ctx, cudaMemcpyAsync(tasks_d, tasks.data(), sizeof(SearchTask) * nt, cudaMemcpyHostToDevice, s));
-    if constexpr (E > 0)
+    if constexpr (E > 0) {
         search_warp_kernel<E><<<blocks, kSearchThreads, 0, s>>>(tasks_d, nt, off_d, st_d, olist_d, rg.nx, rg.ny,
                                                                 part_d);
-    else
+        pick_best_warp<E><<<(nt + 3) / 4, 128, 0, s>>>(rg, tasks_d, nt, part_d, off_d, olist_d, st_d, fix_depth,
+                                                       per_block, best_d);
+    } else {
         search_kernel<NMAX><<<blocks, kSearchThreads, 0, s>>>(tasks_d, nt, off_d, st_d, olist_d, rg.nx, rg.ny,
                                                               part_d);
-    pick_best<NMAX><<<(nt + 127) / 128, 128, 0, s>>>(rg, tasks_d, nt, part_d, off_d, olist_d, st_d, fix_depth,
-                                                     per_block, best_d);
+        pick_best<NMAX><<<(nt + 127) / 128, 128, 0, s>>>(rg, tasks_d, nt, part_d, off_d, olist_d, st_d, fix_depth,
+                                                         per_block, best_d);
+    }
     TS_CUDA_TRY(ctx, cudaGetLastError());
     best.resize(nt);
     TS_CUDA_TRY(ctx, cudaMemcpyAsync(best.data(), best_d, sizeof(int) * nt, cudaMemcpyDeviceToHost, s));
@@ -816,23 +903,25 @@ int run_search(ts_ctx* ctx, const RGrid& rg, std::vector<SearchTask>& tasks, con
 int search_classes(ts_ctx* ctx, const RGrid& rg, const std::vector<SearchTask>& tasks, const std::vector<int>& cls,
                    const int* off_d, EvState* st_d, const ObsD* olist_d, int fix_depth, bool dyadic,
                    std::vector<int>& best_of_event, int64_t& candidates) {
-    for (int c = 0; c < 3; c++) {
+    for (int c = 0; c <= 4; c++) {
         std::vector<SearchTask> part;
         for (const auto& t : tasks)
             if (cls[t.event] == c) part.push_back(t);
         if (part.empty()) continue;
         std::vector<int> best;
-        // Dyadic non-negative weights: one warp per candidate (registers only); otherwise, and above
-        // 128 picks, one thread per candidate.
+        // Dyadic non-negative weights: one warp per candidate with as many picks a lane as the class needs
+        // (registers only); otherwise, and above 128 picks, one thread per candidate.
+        auto warp = [&](auto e) {
+            return run_search<0, decltype(e)::value>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
+        };
         int rc;
-        if (c == 0)
-            rc = dyadic ? run_search<32, 1>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates)
-                        : run_search<32, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
-        else if (c == 1)
-            rc = dyadic ? run_search<128, 4>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates)
-                        : run_search<128, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
-        else
-            rc = run_search<kMaxObs, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
+        if (c == 4) rc = run_search<kMaxObs, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
+        else if (!dyadic && c == 0) rc = run_search<32, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
+        else if (!dyadic) rc = run_search<128, 0>(ctx, rg, part, off_d, st_d, olist_d, fix_depth, best, candidates);
+        else if (c == 0) rc = warp(std::integral_constant<int, 1>());
+        else if (c == 1) rc = warp(std::integral_constant<int, 2>());
+        else if (c == 2) rc = warp(std::integral_constant<int, 3>());
+        else rc = warp(std::integral_constant<int, 4>());
         if (rc) return rc;
         for (size_t k = 0; k < part.size(); k++) best_of_event[part[k].event] = best[k];
     }
