@@ -99,6 +99,8 @@ void ts_cuda_destroy(ts_ctx* ctx) {
         ctx->bufs.clear();
         if (ctx->cancel_host) cudaFreeHost(const_cast<int*>(ctx->cancel_host));
         if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+        for (cudaStream_t s : ctx->copy_streams)
+            if (s) cudaStreamDestroy(s);
         cudaStreamDestroy(ctx->stream);
         // Allocations still held (rows not yet freed) keep the pool's memory until they are freed.
         if (ctx->pool) cudaMemPoolDestroy(ctx->pool);

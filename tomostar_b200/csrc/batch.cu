@@ -9,6 +9,7 @@
 
 #include "ctx.h"
 #include "eik_engine.h"
+#include "host_copy.h"
 #include "host_geo.h"
 
 namespace ts {
@@ -37,15 +38,12 @@ static int solve_multi_impl(ts_ctx* ctx, int n_grids, const ts_grid* grids, cons
     Real* sl = static_cast<Real*>(ctx->buf("multi.slowness", sizeof(Real) * total));
     if (!sl) return TS_E_NOMEM;
     {
-        std::vector<Real> tmp(total);
         size_t o = 0;
         for (int q = 0; q < n_grids; q++) {
             slow_d[q] = sl + o;
-            for (int64_t e = 0; e < g[q]->count(); e++) tmp[o + e] = Real(slowness[q][e]);
+            if (int rc = upload_values(ctx, slow_d[q], slowness[q], size_t(g[q]->count()), ctx->stream)) return rc;
             o += size_t(g[q]->count());
         }
-        TS_CUDA_TRY(ctx, cudaMemcpyAsync(sl, tmp.data(), sizeof(Real) * total, cudaMemcpyHostToDevice, ctx->stream));
-        TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     }
     job.tol = tol;
     job.wake_rel = mode == TS_MODE_FAST ? TS_WAKE_REL : 0.0;

@@ -16,6 +16,9 @@ struct ts_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // device→host copies that overlap the next solve (created on use)
+    // Streams of the threads of a pageable copy (host_copy.cu; created on use).
+    static constexpr int kCopyStreams = 8;
+    cudaStream_t copy_streams[kCopyStreams] = {};
     std::recursive_mutex mu;  // calls on one context are serialised (EikonalOpenCl.cs:64,165)
     std::string err;
     std::string stats;

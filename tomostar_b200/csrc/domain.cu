@@ -11,6 +11,7 @@
 
 #include "ctx.h"
 #include "geo_dev.cuh"
+#include "host_copy.h"
 #include "host_geo.h"
 
 namespace ts {
@@ -249,7 +250,7 @@ int ts_model_copy_slowness(ts_ctx* ctx, int32_t model_id, int32_t phase, double*
     if (phase < 0 || phase >= m->n_phases) return ctx->fail(TS_E_ARG, "phase out of range");
     const size_t n = size_t(m->grid->count());
     if (m->precision == TS_PRECISION_F64) {
-        TS_CUDA_TRY(ctx, cudaMemcpy(out, static_cast<double*>(m->slowness) + n * phase, n * 8, cudaMemcpyDeviceToHost));
+        if (int rc = ts::copy_to_host(ctx, out, static_cast<double*>(m->slowness) + n * phase, n * 8, ctx->stream)) return rc;
     } else {
         // The FP32 precision's slowness is the float the paired kernel reads (the pair's hi).
         std::vector<Pair> tmp(n);

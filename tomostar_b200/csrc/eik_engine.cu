@@ -2,11 +2,13 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "eik_engine.h"
 #include "eik_kernels.cuh"
 #include "eik_resident.h"
+#include "host_copy.h"
 
 namespace ts {
 namespace eik {
@@ -40,71 +42,86 @@ static int tile_for(const ts_ctx* ctx, const EngineJob& job) {
 
 namespace {
 
-// Padded engine fields → dense grid order of another precision (one field per blockIdx.y).
+// A padded engine field → dense grid order, of another type with non-finite values as +inf, or of its own
+// as it is. A warp per row.
 template <typename From, typename To>
-__global__ void dense_convert_kernel(const From* __restrict__ a, int64_t field_stride, int pitch, int xoff, int nx,
-                                     int64_t rows, To* __restrict__ b) {
-    const From* src = a + blockIdx.y * field_stride;
-    To* dst = b + int64_t(blockIdx.y) * rows * nx;
-    for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < rows * nx; q += int64_t(gridDim.x) * blockDim.x) {
-        int64_t r = q / nx;
-        From v = src[r * pitch + xoff + (q - r * nx)];
-        dst[q] = finite_r(v) ? To(v) : To(__int_as_float(0x7f800000));
+__global__ void dense_convert_kernel(const From* __restrict__ a, int pitch, int xoff, int nx, int64_t rows,
+                                     To* __restrict__ b) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = int64_t(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t r = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; r < rows; r += nw) {
+        const From* src = a + r * pitch + xoff;
+        To* dst = b + r * nx;
+        for (int q = lane; q < nx; q += 32) {
+            const From v = src[q];
+            if constexpr (std::is_same_v<From, To>) dst[q] = v;
+            else dst[q] = finite_r(v) ? To(v) : To(__int_as_float(0x7f800000));
+        }
     }
+}
+
+// One padded field on a grid to dense values of out_type at out (device), on s.
+template <typename Real>
+cudaError_t field_to_dense(const Real* T, const host::Grid& g, int pitch, int xoff, void* out, int out_type, cudaStream_t s) {
+    const int64_t rows = int64_t(g.ny) * g.nz;
+    const int blocks = int(std::min<int64_t>((rows + 7) / 8, 4096));
+    if (out_type == TS_OUT_F64)
+        dense_convert_kernel<Real, double><<<blocks, 256, 0, s>>>(T, pitch, xoff, g.nx, rows, static_cast<double*>(out));
+    else
+        dense_convert_kernel<Real, float><<<blocks, 256, 0, s>>>(T, pitch, xoff, g.nx, rows, static_cast<float*>(out));
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-// Fields of the job in dense grid order: same precision → strided copies; otherwise converted on the
-// device in blocks of fields, then copied.
-int fields_to_dense_host(ts_ctx* ctx, const EngineJob& job, int precision, void* out, int out_type) {
-    const size_t rsz = 8;  // a double, or the FP32 precision's float pair
+// Fields [f0, f1) of a job (after engine_run) in dense grid order of out_type, one after another at dst, on s.
+template <typename Real>
+static int fields_to_dense_device(ts_ctx* ctx, const EngineJob& job, size_t f0, size_t f1, void* dst, int out_type,
+                                  cudaStream_t s) {
+    char* d = static_cast<char*>(dst);
     const size_t osz = out_type == TS_OUT_F64 ? 8 : 4;
-    const bool same = precision == TS_PRECISION_F64 && out_type == TS_OUT_F64;
-    char* dst = static_cast<char*>(out);
-    for (size_t f = 0; f < job.fields.size(); f++) {
+    for (size_t f = f0; f < f1; f++) {
         const host::Grid& g = *job.grids[job.fields[f].grid];
-        const int pitch = job.pitch[job.fields[f].grid];
-        const int64_t rows = int64_t(g.ny) * g.nz, n = rows * g.nx;
-        const char* src = static_cast<const char*>(job.fields[f].T);
-        if (same) {
-            TS_CUDA_TRY(ctx, cudaMemcpy2DAsync(dst, g.nx * osz, src + job.xoff * rsz, pitch * rsz, g.nx * rsz, rows,
-                                               cudaMemcpyDeviceToHost, ctx->stream));
-        } else {
-            void* stage = ctx->buf("out.stage", size_t(n) * osz);
-            if (!stage) return TS_E_NOMEM;
-            int blocks = int(std::min<int64_t>((n + 255) / 256, 4096));
-            if (precision == TS_PRECISION_F64)
-                dense_convert_kernel<double, float><<<dim3(blocks, 1), 256, 0, ctx->stream>>>(
-                    reinterpret_cast<const double*>(src), 0, pitch, job.xoff, g.nx, rows, static_cast<float*>(stage));
-            else if (osz == 8)
-                dense_convert_kernel<Pair, double><<<dim3(blocks, 1), 256, 0, ctx->stream>>>(
-                    reinterpret_cast<const Pair*>(src), 0, pitch, job.xoff, g.nx, rows, static_cast<double*>(stage));
-            else
-                dense_convert_kernel<Pair, float><<<dim3(blocks, 1), 256, 0, ctx->stream>>>(
-                    reinterpret_cast<const Pair*>(src), 0, pitch, job.xoff, g.nx, rows, static_cast<float*>(stage));
-            TS_CUDA_TRY(ctx, cudaGetLastError());
-            TS_CUDA_TRY(ctx, cudaMemcpyAsync(dst, stage, size_t(n) * osz, cudaMemcpyDeviceToHost, ctx->stream));
-            TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        }
-        dst += size_t(n) * osz;
+        TS_CUDA_TRY(ctx, field_to_dense(static_cast<const Real*>(job.fields[f].T), g, job.pitch[job.fields[f].grid],
+                                        job.xoff, d, out_type, s));
+        d += size_t(g.count()) * osz;
     }
-    TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    return TS_OK;
+}
+
+// Fields of the job to the host in dense grid order: made dense on the device in runs of fields, each run
+// copied at once.
+int fields_to_dense_host(ts_ctx* ctx, const EngineJob& job, int precision, void* out, int out_type) {
+    const size_t osz = out_type == TS_OUT_F64 ? 8 : 4, most = size_t(512) << 20;
+    char* dst = static_cast<char*>(out);
+    for (size_t f0 = 0; f0 < job.fields.size();) {
+        size_t f1 = f0, bytes = 0;
+        while (f1 < job.fields.size()) {
+            const size_t b = size_t(job.grids[job.fields[f1].grid]->count()) * osz;
+            if (f1 > f0 && bytes + b > most) break;
+            bytes += b;
+            f1++;
+        }
+        void* stage = ctx->buf("out.stage", bytes);
+        if (!stage) return TS_E_NOMEM;
+        int rc = precision == TS_PRECISION_F64
+                     ? fields_to_dense_device<double>(ctx, job, f0, f1, stage, out_type, ctx->stream)
+                     : fields_to_dense_device<Pair>(ctx, job, f0, f1, stage, out_type, ctx->stream);
+        if (rc == TS_OK) rc = copy_to_host(ctx, dst, stage, bytes, ctx->stream);
+        if (rc) return rc;
+        dst += bytes;
+        f0 = f1;
+    }
     return TS_OK;
 }
 
 // One field as a dense float32 table on the device (the .qttb rounding).
 int field_to_dense_f32_device(ts_ctx* ctx, const host::Grid& g, const FieldLayout& L, const void* T, int precision,
                               float* out, cudaStream_t s) {
-    const int64_t rows = int64_t(g.ny) * g.nz, n = rows * g.nx;
-    int blocks = int(std::min<int64_t>((n + 255) / 256, 2048));
     if (precision == TS_PRECISION_F64)
-        dense_convert_kernel<double, float><<<dim3(blocks, 1), 256, 0, s>>>(static_cast<const double*>(T), 0, L.pitch,
-                                                                            L.xoff, g.nx, rows, out);
+        TS_CUDA_TRY(ctx, field_to_dense(static_cast<const double*>(T), g, L.pitch, L.xoff, out, TS_OUT_F32, s));
     else
-        dense_convert_kernel<Pair, float><<<dim3(blocks, 1), 256, 0, s>>>(static_cast<const Pair*>(T), 0, L.pitch,
-                                                                          L.xoff, g.nx, rows, out);
-    TS_CUDA_TRY(ctx, cudaGetLastError());
+        TS_CUDA_TRY(ctx, field_to_dense(static_cast<const Pair*>(T), g, L.pitch, L.xoff, out, TS_OUT_F32, s));
     return TS_OK;
 }
 
@@ -186,30 +203,6 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     if (!chosen && !ctx->use_graph)
         if (const int cluster = resident_cluster(ctx, job)) return resident_run<Real>(ctx, job, cluster, stats, ctx->stream);
     return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, job.tile, 0, stats, ctx->stream);
-}
-
-// Fields [f0, f1) of a job (after engine_run) converted to dense grid order of out_type into dst, on s.
-template <typename Real>
-static int fields_to_dense_device(ts_ctx* ctx, const EngineJob& job, size_t f0, size_t f1, void* dst, int out_type,
-                                  cudaStream_t s) {
-    char* d = static_cast<char*>(dst);
-    const size_t osz = out_type == TS_OUT_F64 ? 8 : 4;
-    for (size_t f = f0; f < f1; f++) {
-        const host::Grid& g = *job.grids[job.fields[f].grid];
-        const int pitch = job.pitch[job.fields[f].grid];
-        const int64_t rows = int64_t(g.ny) * g.nz, n = rows * g.nx;
-        const int blocks = int(std::min<int64_t>((n + 255) / 256, 4096));
-        const Real* src = static_cast<const Real*>(job.fields[f].T);
-        if (osz == 8)
-            dense_convert_kernel<Real, double><<<dim3(blocks, 1), 256, 0, s>>>(src, 0, pitch, job.xoff, g.nx, rows,
-                                                                               reinterpret_cast<double*>(d));
-        else
-            dense_convert_kernel<Real, float><<<dim3(blocks, 1), 256, 0, s>>>(src, 0, pitch, job.xoff, g.nx, rows,
-                                                                              reinterpret_cast<float*>(d));
-        TS_CUDA_TRY(ctx, cudaGetLastError());
-        d += size_t(n) * osz;
-    }
-    return TS_OK;
 }
 
 template <typename Real>

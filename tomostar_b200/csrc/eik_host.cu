@@ -9,6 +9,7 @@
 #include "ctx.h"
 #include "eik_engine.h"
 #include "eik_kernels.cuh"
+#include "host_copy.h"
 #include "host_geo.h"
 
 namespace ts {
@@ -173,14 +174,11 @@ int model_put(ts_ctx* ctx, const ts_grid* grid, const double* slowness, int n_ph
         return ctx->fail(TS_E_NOMEM, "model slowness");
     }
     int rc = TS_OK;
-    if (precision == TS_PRECISION_F64) {
-        if (cudaMemcpy(m->slowness, slowness, count * 8, cudaMemcpyHostToDevice) != cudaSuccess) rc = TS_E_CUDA;
-    } else {
-        std::vector<Pair> tmp(count);
-        for (size_t q = 0; q < count; q++) tmp[q] = Pair(slowness[q]);
-        if (cudaMemcpy(m->slowness, tmp.data(), count * sizeof(Pair), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = TS_E_CUDA;
-    }
+    if (precision == TS_PRECISION_F64)
+        rc = upload_values(ctx, static_cast<double*>(m->slowness), slowness, count, ctx->stream);
+    else
+        rc = upload_values(ctx, static_cast<Pair*>(m->slowness), slowness, count, ctx->stream);
+    if (rc == TS_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = TS_E_CUDA;
     if (rc) {
         delete m;
         return ctx->fail(rc, "model upload");
@@ -240,7 +238,11 @@ static int solve_impl(ts_ctx* ctx, const SolveIn& in, void* out, int out_type, t
     Real* slow_d;
     int rc = TS_OK;
     if (model) slow_d = static_cast<Real*>(model->slowness) + size_t(n) * in.phase;
-    else if ((rc = upload_real<Real>(ctx, "solve.slowness", in.slowness, size_t(n), &slow_d))) return rc;
+    else {
+        slow_d = static_cast<Real*>(ctx->buf("solve.slowness", sizeof(Real) * size_t(n)));
+        if (!slow_d) return TS_E_NOMEM;
+        if ((rc = upload_values(ctx, slow_d, in.slowness, size_t(n), ctx->stream))) return rc;
+    }
     const int cap = in.max_rounds > 0 ? in.max_rounds : std::max(32, (g.nx + g.ny + g.nz) / 4);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);

@@ -11,20 +11,12 @@
 
 #include "ctx.h"
 #include "eik_engine.h"
+#include "host_copy.h"
 #include "host_geo.h"
 #include "rays.h"
 
 namespace ts {
 namespace fwd {
-
-template <typename Real>
-static int upload_slowness(ts_ctx* ctx, const double* src, size_t count, Real* dst) {
-    std::vector<Real> tmp(count);
-    for (size_t q = 0; q < count; q++) tmp[q] = Real(src[q]);
-    TS_CUDA_TRY(ctx, cudaMemcpyAsync(dst, tmp.data(), count * sizeof(Real), cudaMemcpyHostToDevice, ctx->stream));
-    TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    return TS_OK;
-}
 
 // The float32 tables of `tables` ((phase, source) pairs; sources hold lon, lat, depth) on g, solved
 // by the engine in batches that fit the device next to the tables, each rounded to float32 into its
@@ -41,7 +33,7 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
     // Slowness per phase on the device.
     Real* slow_d = static_cast<Real*>(ctx->buf("fwd.slowness", sizeof(Real) * size_t(n) * n_phases));
     if (!slow_d) return TS_E_NOMEM;
-    int rc = upload_slowness<Real>(ctx, slowness, size_t(n) * n_phases, slow_d);
+    int rc = upload_values(ctx, slow_d, slowness, size_t(n) * n_phases, ctx->stream);
     if (rc) return rc;
     // Seeds: PointSource at each source (TravelTimeTable.cs:373).
     std::vector<std::vector<int32_t>> sidx(nt);
@@ -127,7 +119,9 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
     }
     ctx->stats = std::to_string(r0) + "+" + std::to_string(r1) + " rounds of 8 sweeps";
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    ctx->release("eng.fields");
+    // Small field buffers stay for the next call (mapping and unmapping 4 GB takes 5 ms, on a device in use
+    // up to hundreds); large ones make room for the rows.
+    if (ctx->bufs["eng.fields"].n > ctx->total_mem / 8) ctx->release("eng.fields");
     return TS_OK;
 }
 

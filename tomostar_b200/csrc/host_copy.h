@@ -1,0 +1,20 @@
+// Copies between the caller's pageable memory and the device.
+#pragma once
+
+#include "ctx.h"
+#include "ts_common.cuh"
+
+namespace ts {
+
+// bytes from device src, as stream s leaves it, to host dst; returns when dst holds them.
+int copy_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+// bytes from host src to device dst, after what stream s has queued; work queued on s afterwards sees
+// them, and src may change when the call returns.
+int copy_to_device(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+// count doubles of the host as FP64 values, or as the FP32 precision's float pairs (formed on the device).
+int upload_values(ts_ctx* ctx, double* dst, const double* src, size_t count, cudaStream_t s);
+int upload_values(ts_ctx* ctx, Pair* dst, const double* src, size_t count, cudaStream_t s);
+
+}  // namespace ts

@@ -20,6 +20,7 @@
 
 #include "ctx.h"
 #include "geo_dev.cuh"
+#include "host_copy.h"
 #include "host_geo.h"
 #include "tables.h"
 
@@ -946,15 +947,15 @@ int ts_tables_upload(ts_ctx* ctx, const ts_grid* grid, int32_t n_tables, const f
     t->n_tables = n_tables;
     t->nodes = int64_t(grid->nx) * grid->ny * grid->nz;
     const size_t bytes = sizeof(float) * size_t(t->nodes) * size_t(n_tables);
-    if (cudaMalloc(&t->dev, bytes) != cudaSuccess) {
+    if (ctx->alloc_async(&t->dev, bytes, ctx->stream) != cudaSuccess) {
         cudaGetLastError();
         delete t;
         return ctx->fail(TS_E_NOMEM, "no device memory for the tables");
     }
-    if (cudaMemcpy(t->dev, tables, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(t->dev);
+    if (int rc = copy_to_device(ctx, t->dev, tables, bytes, ctx->stream)) {
+        cudaFreeAsync(t->dev, ctx->stream);
         delete t;
-        return ctx->fail(TS_E_CUDA, "table upload failed");
+        return rc;
     }
     *out = t;
     return TS_OK;
@@ -982,7 +983,7 @@ int ts_tables_build(ts_ctx* ctx, const ts_grid* grid, const double* slowness, in
     tb->def = *grid;
     tb->n_tables = n_tables;
     tb->nodes = int64_t(grid->nx) * grid->ny * grid->nz;
-    if (cudaMalloc(&tb->dev, sizeof(float) * size_t(tb->nodes) * size_t(n_tables)) != cudaSuccess) {
+    if (ctx->alloc_async(&tb->dev, sizeof(float) * size_t(tb->nodes) * size_t(n_tables), ctx->stream) != cudaSuccess) {
         cudaGetLastError();
         delete tb;
         return ctx->fail(TS_E_NOMEM, "no device memory for the tables");
@@ -994,7 +995,7 @@ int ts_tables_build(ts_ctx* ctx, const ts_grid* grid, const double* slowness, in
                  ? fwd::solve_tables<double>(ctx, g, slowness, n_phases, TS_MODE_ENGINE, list, sources, tb->dev, stats)
                  : ctx->fail(TS_E_ARG, "precision must be 64 or 32");
     if (rc) {
-        cudaFree(tb->dev);
+        cudaFreeAsync(tb->dev, ctx->stream);
         delete tb;
         return rc;
     }
@@ -1014,8 +1015,7 @@ int ts_tables_copy(ts_tables* t, int32_t first, int32_t count, float* out) {
     std::lock_guard<std::recursive_mutex> lk(t->ctx->mu);
     cudaSetDevice(t->ctx->device);
     const size_t n = size_t(t->nodes);
-    TS_CUDA_TRY(t->ctx, cudaMemcpy(out, t->dev + n * first, sizeof(float) * n * count, cudaMemcpyDeviceToHost));
-    return TS_OK;
+    return copy_to_host(t->ctx, out, t->dev + n * first, sizeof(float) * n * count, t->ctx->stream);
 }
 
 void ts_tables_free(ts_tables* t) {
@@ -1023,7 +1023,7 @@ void ts_tables_free(ts_tables* t) {
     {
         std::lock_guard<std::recursive_mutex> lk(t->ctx->mu);
         cudaSetDevice(t->ctx->device);
-        cudaFree(t->dev);
+        cudaFreeAsync(t->dev, t->ctx->stream);
     }
     delete t;
 }

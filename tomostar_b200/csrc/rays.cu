@@ -28,6 +28,7 @@
 
 #include "ctx.h"
 #include "geo_dev.cuh"
+#include "host_copy.h"
 #include "host_geo.h"
 #include "rays.h"
 
@@ -994,7 +995,7 @@ int ts_rays_trace(ts_ctx* ctx, const ts_grid* fwd, int32_t n_tables, const float
     const size_t bytes = sizeof(float) * size_t(n_tables) * size_t(gf.count());
     float* d_tables = static_cast<float*>(ctx->buf("rays.tables", bytes));
     if (!d_tables) return TS_E_NOMEM;
-    TS_CUDA_TRY(ctx, cudaMemcpyAsync(d_tables, tables, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if (int rc = copy_to_device(ctx, d_tables, tables, bytes, ctx->stream)) return rc;
     return ts::rays::trace_on_device(ctx, gf, d_tables, n_tables, table_station, gi, n_rays, table_of, events, step_km,
                                      out, nullptr);
 }
@@ -1014,9 +1015,11 @@ int ts_rows_copy(ts_rows* rows, int32_t* row_ptr, int32_t* col, float* len, doub
     cudaStream_t s = ctx->stream;
     const int n = rows->n_rows;
     if (row_ptr) TS_CUDA_TRY(ctx, cudaMemcpyAsync(row_ptr, rows->row_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, s));
-    if (col && rows->nnz) TS_CUDA_TRY(ctx, cudaMemcpyAsync(col, rows->col, sizeof(int) * rows->nnz, cudaMemcpyDeviceToHost, s));
-    if (len && rows->nnz) TS_CUDA_TRY(ctx, cudaMemcpyAsync(len, rows->len, sizeof(float) * rows->nnz, cudaMemcpyDeviceToHost, s));
     if (tcalc_grad && n) TS_CUDA_TRY(ctx, cudaMemcpyAsync(tcalc_grad, rows->tcg, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s));
+    if (col && rows->nnz)
+        if (int rc = copy_to_host(ctx, col, rows->col, sizeof(int) * size_t(rows->nnz), s)) return rc;
+    if (len && rows->nnz)
+        if (int rc = copy_to_host(ctx, len, rows->len, sizeof(float) * size_t(rows->nnz), s)) return rc;
     if (ok && n) TS_CUDA_TRY(ctx, cudaMemcpyAsync(ok, rows->ok, size_t(n), cudaMemcpyDeviceToHost, s));
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     return TS_OK;

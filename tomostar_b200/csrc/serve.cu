@@ -28,6 +28,7 @@
 
 #include "ctx.h"
 #include "eik_engine.h"
+#include "host_copy.h"
 #include "host_geo.h"
 #include "rays.h"
 #include "ts_common.cuh"
@@ -272,13 +273,9 @@ void complete_batch(ts_server* sv, const std::vector<ServeRequest*>& reqs, std::
         ServeRequest* r = reqs[k];
         if (codes[k] != TS_OK || !r->tables_out) continue;
         const int64_t n = ctx->models.at(r->model_id)->grid->count();
-        cudaError_t e = cudaMemcpyAsync(r->tables_out, r->tables_dev, sizeof(float) * size_t(n) * r->n_fields,
-                                        cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            codes[k] = TS_E_CUDA;
-            errors[k] = cudaGetErrorString(e);
-        }
+        const int rc = ts::copy_to_host(ctx, r->tables_out, r->tables_dev, sizeof(float) * size_t(n) * r->n_fields,
+                                        ctx->stream);
+        if (rc) fail(k, rc);
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
