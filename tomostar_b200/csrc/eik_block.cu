@@ -28,10 +28,9 @@ struct Arena {
 
 // New fields of an epoch: +inf everywhere (pads included), every tile and node due, state zero.
 template <typename Real>
-__global__ void init_fields_kernel(const FieldDesc<Real>* __restrict__ fields, const GridDesc* __restrict__ grids,
-                                   const int* __restrict__ init_list, int mw) {
+__global__ void init_fields_kernel(const FieldDesc<Real>* __restrict__ fields, const int* __restrict__ init_list, int mw) {
     const FieldDesc<Real>& fd = fields[init_list[blockIdx.y]];
-    const GridDesc& g = grids[fd.grid];
+    const GridDesc& g = fd.g;
     int64_t n = int64_t(g.pitch) * g.ny * g.nz;
     const Real inf = real_inf<Real>();
     const int64_t t0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
@@ -43,13 +42,12 @@ __global__ void init_fields_kernel(const FieldDesc<Real>* __restrict__ fields, c
 }
 
 template <typename Real>
-__global__ void seed_fields_kernel(const FieldDesc<Real>* __restrict__ fields, const GridDesc* __restrict__ grids,
-                                   const int* __restrict__ field_of, const int32_t* __restrict__ node,
+__global__ void seed_fields_kernel(const FieldDesc<Real>* __restrict__ fields, const int* __restrict__ field_of, const int32_t* __restrict__ node,
                                    const double* __restrict__ t, int count) {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= count) return;
     const FieldDesc<Real>& fd = fields[field_of[q]];
-    const GridDesc& g = grids[fd.grid];
+    const GridDesc& g = fd.g;
     int n = node[q], i = n % g.nx, row = n / g.nx;
     fd.T[int64_t(row) * g.pitch + Layout<Real>::HX + i] = Real(t[q]);
 }
@@ -68,6 +66,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     constexpr int BX = kTileX;
     using B = BlockTile<Real, BX, BY, BZ>;
     const int nf = int(fl.size());
+    if (nf >= kMaxFields) return ctx->fail(TS_E_ARG, "too many fields in one launch");
     const int ng = int(grids.size());
     bool any_var = false;
     for (auto* g : grids) any_var |= g->variable;
@@ -76,7 +75,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     // Grids.
     std::vector<size_t> o_diag_off(ng), o_diag_tiles(ng), o_wx(ng), o_wy(ng), o_zc(ng);
     std::vector<int> tx(ng), ty(ng), tz(ng), ndiag(ng);
-    size_t o_grids = A.add(sizeof(GridDesc) * ng);
+    std::vector<GridDesc> descs(ng);
     for (int gi = 0; gi < ng; gi++) {
         const host::Grid& g = *grids[gi];
         const host::Metric& m = *metrics[gi];
@@ -193,9 +192,8 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
 
     uint8_t* D = static_cast<uint8_t*>(ctx->buf("eng.arena", A.h.size()));
     if (!D) return TS_E_NOMEM;
-    auto* q_items = static_cast<unsigned long long*>(ctx->buf("eng.q_items", 8 * qcap));
-    auto* q_seq = static_cast<unsigned long long*>(ctx->buf("eng.q_seq", 8 * qcap));
-    if (!q_items || !q_seq) return TS_E_NOMEM;
+    auto* q_slots = static_cast<unsigned long long*>(ctx->buf("eng.q_slots", 8 * qcap));
+    if (!q_slots) return TS_E_NOMEM;
     for (int gi = 0; gi < ng; gi++) {
         GridDesc gd{};
         const host::Grid& g = *grids[gi];
@@ -211,7 +209,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
         gd.wz1 = weight_of<Real>(metrics[gi]->wz1, metrics[gi]->wz1_32);
         gd.wz2 = weight_of<Real>(metrics[gi]->wz2, metrics[gi]->wz2_32);
         gd.pitch = Layout<Real>::pitch(tx[gi], BX);
-        A.at<GridDesc>(o_grids)[gi] = gd;
+        descs[gi] = gd;
     }
     for (int f = 0; f < nf; f++) {
         const EngineField& ef = *fl[f];
@@ -220,7 +218,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
         fd.s = static_cast<const Real*>(ef.slowness);
         fd.dirty = ef.dirty;
         fd.dmask = ef.dmask;
-        fd.grid = ef.grid;
+        fd.g = descs[ef.grid];
         fd.seed_begin = seed_begin[f];
         fd.seed_count = seed_count[f];
         fd.cap = ef.cap;
@@ -243,7 +241,6 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     *ctl_h = Control{};
 
     Args<Real> args{};
-    args.grids = reinterpret_cast<const GridDesc*>(D + o_grids);
     args.fields = reinterpret_cast<const FieldDesc<Real>*>(D + o_fields);
     args.seed_tile = reinterpret_cast<const int*>(D + o_seed_tile);
     args.seed_mask = reinterpret_cast<const uint32_t*>(D + o_seed_mask);
@@ -254,9 +251,9 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     args.max_rounds_per_launch = max_rounds;
     args.epoch_budget_ns = (ctx->scheduler == 1 && max_rounds > 0) ? (long long)(ctx->epoch_budget_ms * 1e6) : 0;
     args.barrier_timeout_ns = 5000000000LL;
-    args.q_items = q_items;
-    args.q_seq = q_seq;
+    args.q_slots = q_slots;
     args.q_mask = qcap - 1;
+    for (args.q_bits = 0; (size_t(1) << args.q_bits) < qcap;) args.q_bits++;
     args.tol = Real(tol);
     args.wake_rel = Real(wake_rel);
     args.causal = wake_rel > 0 ? 1 : 0;  // fast mode: threshold and causal wakes together
@@ -282,20 +279,15 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
             unsigned cnt = unsigned(std::min<size_t>(65535, init_list.size() - c0));
             dim3 grid(unsigned(std::min<int64_t>((maxn + 255) / 256, 512)), cnt);
             init_fields_kernel<Real><<<grid, 256, 0, s>>>(reinterpret_cast<const FieldDesc<Real>*>(D + o_fields),
-                                                          reinterpret_cast<const GridDesc*>(D + o_grids),
                                                           reinterpret_cast<const int*>(D + o_init) + c0, B::MW);
         }
         int cnt = int(sc_node.size());
         if (cnt > 0)
             seed_fields_kernel<Real><<<(cnt + 255) / 256, 256, 0, s>>>(
-                reinterpret_cast<const FieldDesc<Real>*>(D + o_fields), reinterpret_cast<const GridDesc*>(D + o_grids),
-                reinterpret_cast<const int*>(D + o_sc_field), reinterpret_cast<const int32_t*>(D + o_sc_node),
+                reinterpret_cast<const FieldDesc<Real>*>(D + o_fields), reinterpret_cast<const int*>(D + o_sc_field), reinterpret_cast<const int32_t*>(D + o_sc_node),
                 reinterpret_cast<const double*>(D + o_sc_t), cnt);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if (running > 0) {
-            flow_queue_init<<<int(std::min<size_t>((qcap + 255) / 256, 1024)), 256, 0, s>>>(q_seq, qcap);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        }
+        if (running > 0 && (e = cudaMemsetAsync(q_slots, 0, 8 * qcap, s)) != cudaSuccess) return e;
         if (running > 0) {
             if (timed) cudaEventRecord(k0, s);
             e = cudaLaunchCooperativeKernel(kfn, dim3(blocks), dim3(B::kThreads), params, smem, s);
@@ -317,7 +309,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
             for (size_t q = 0; q < n; q++) sig = (sig ^ b[q]) * 1099511628211ULL;
         };
         mix(A.h.data(), A.h.size());
-        uintptr_t ptrs[4] = {uintptr_t(D), uintptr_t(q_items), uintptr_t(image), uintptr_t(kfn)};
+        uintptr_t ptrs[4] = {uintptr_t(D), uintptr_t(q_slots), uintptr_t(image), uintptr_t(kfn)};
         mix(ptrs, sizeof ptrs);
         if (ctx->graph_exec && ctx->graph_sig == sig) {
             TS_CUDA_TRY(ctx, cudaGraphLaunch(ctx->graph_exec, s));

@@ -7,9 +7,10 @@
 // diagonals of 44 steps. Here the tile and its two-node halo lie in shared memory in grid orientation, so
 // a step is 13 loads at fixed offsets from one address, the update, one store and a byte per woken node;
 // the field is crossed in 18 diagonals of 54 steps (32×16×8) or 14 of 62 (32×16×16). Measured against the
-// better of the earlier shapes (kernel time): 50 fields of 121×121×61 162 -> 75 ms, 10 of 161×161×81
-// (every drop wakes) 292 -> 133, 25 of 81×81×41 64 -> 28, 24 of 401×401×121 1,205 -> 816, 400 of
-// 101×101×61 341 -> 299.
+// better of the earlier shapes (kernel time): 50 fields of 121×121×61 162 -> 60 ms, 10 of 161×161×81
+// (every drop wakes) 292 -> 117, 25 of 81×81×41 64 -> 24, 24 of 401×401×121 1,205 -> 673, 400 of
+// 101×101×61 341 -> 244. A plane with due nodes takes some 1,500 cycles, 850 of them the update's chain;
+// a visit's load, write-back and hand-over some 15,000, as much as ten planes.
 //
 // Inside a tile the reference's plane order i'+j'+k' = p (mirrored coordinates) is kept: at step p the
 // thread of canonical row (j', k') evaluates the node i' = p − j' − k', one block barrier per step. A
@@ -53,7 +54,6 @@ constexpr int kMaxRowWaits = 1 << 20;
 struct BlockShared {  // the last 64 bytes of the block's shared memory
     unsigned long long entry;
     unsigned long long arrived;  // mbarrier of the tile's row copies
-    int state, pad;
     int first[8];  // per warp: the first plane with a due node
 };
 
@@ -83,11 +83,14 @@ TS_DEVINL bool rows_arrived(unsigned bar, unsigned parity) {
     return ok != 0;
 }
 
-// Visits one tile of one field for sweep ordering `dir`; the whole block. Returns the thread's node
+// Visits one tile of one field for its sweep ordering; the whole block. Returns the thread's node
 // evaluations.
 template <typename Real, int BX, int BY, int BZ, bool VARZ>
-TS_DEVINL int visit_block(const Args<Real>& a, const GridDesc& g, const FieldDesc<Real>& fd, int tx, int ty, int tz,
-                          int dir, bool second, unsigned char* smem, BlockShared* sh, unsigned parity) {
+TS_DEVINL int visit_block(const Args<Real>& a, const FieldDesc<Real>& fd, const TileItem& it, unsigned char* smem,
+                          BlockShared* sh, unsigned parity) {
+    const GridDesc& g = fd.g;
+    const int tx = it.tx, ty = it.ty, tz = it.tz, dir = it.dir;
+    const bool second = it.phase == 1;
     using B = BlockTile<Real, BX, BY, BZ>;
     constexpr int P = B::PITCH, L = B::LEVEL, RY = B::RY;
     Real* const T = reinterpret_cast<Real*>(smem) - 2 * P;
@@ -184,8 +187,6 @@ TS_DEVINL int visit_block(const Args<Real>& a, const GridDesc& g, const FieldDes
 
     const Real tol = a.tol, wake_rel = a.wake_rel;
     const bool causal = a.causal != 0;
-    const int xlast = min(BX, nx - x0) - 1;  // last on-grid node of the row
-    auto lds = [&](int ip) -> Real { return ldg_r(srow + max(0, min(mx ? BX - 1 - ip : ip, xlast))); };
     // The first plane that holds a due node: nothing can be woken before it.
     int p = B::NSTEPS;
 #pragma unroll
@@ -194,23 +195,27 @@ TS_DEVINL int visit_block(const Args<Real>& a, const GridDesc& g, const FieldDes
     const int wlo = __reduce_min_sync(0xffffffffu, off), whi = __reduce_max_sync(0xffffffffu, off) + BX - 1;
     bool big = false, mod = false;
     int evals = 0, woke = -4;  // woke: the last plane in which the thread woke a node
-    // Slowness four steps ahead.
-    const int ps = max(p, wlo) - off;
-    Real s1 = lds(ps), s2 = lds(ps + 1), s3 = lds(ps + 2), s4 = lds(ps + 3);
+    // The thread's node of the plane and what lies at it move one node per plane.
+    const int di = mx ? -1 : 1;
+    int i = mx ? BX - 1 + off - p : p - off;  // off the row outside [0, BX)
+    Real* c = T + slot * P + B::HX + i;
+    uint8_t* d = due + slot * DP + 4 + i;
+    // Slowness two planes ahead, where the row has a node then.
+    const int xn = row_on ? min(BX, nx - x0) : 0;
+    const Real* sp = srow + i;
+    auto slow_at = [&](int q) -> Real { return unsigned(i + q * di) < unsigned(xn) ? ldg_r(sp + q * di) : Real(0); };
+    const int skip = max(wlo - p, 0);  // to the warp's first plane
+    Real s1 = slow_at(skip), s2 = slow_at(skip + 1);
+    // A wake reaches the neighbours holding more than the new time (causal rule), or all.
+    const Real none = minus_inf<Real>();
     for (; p < B::NSTEPS; p++) {
-        const int ip = p - off;
+        const Real s0 = s1;
         if (p >= wlo && p <= whi) {
-            const Real s0 = s1;
             s1 = s2;
-            s2 = s3;
-            s3 = s4;
-            s4 = lds(ip + 4);
-            const int i = mx ? BX - 1 - ip : ip;
-            uint8_t* const d = due + slot * DP + 4 + i;
-            if (unsigned(ip) < unsigned(BX) && *(volatile uint8_t*)d && !((fixed >> i) & 1u)) {
+            s2 = slow_at(2);
+            if (unsigned(i) < unsigned(BX) && *(volatile uint8_t*)d && !((fixed >> i) & 1u)) {
                 *d = 0;
                 evals++;
-                Real* const c = T + slot * P + B::HX + i;
                 const Real cur = c[0];
                 const Real xm = c[-1], xp = c[1], xm2 = c[-2], xp2 = c[2];
                 const Real ym = c[-P], yp = c[P], ym2 = c[-2 * P], yp2 = c[2 * P];
@@ -222,29 +227,33 @@ TS_DEVINL int visit_block(const Args<Real>& a, const GridDesc& g, const FieldDes
                     mod = true;
                     if (counts_as_change<Real>(cur, cand, tol)) big = true;
                     if (wakes<Real>(cur, cand, wake_rel)) {
-                        // The 12 stencil neighbours; with the causal rule those holding more than cand.
-                        auto w = [&](Real v) { return !causal || cand < v; };
+                        const Real over = causal ? cand : none;
                         woke = p;
-                        if (w(xm)) d[-1] = 1;
-                        if (w(xp)) d[1] = 1;
-                        if (w(xm2)) d[-2] = 1;
-                        if (w(xp2)) d[2] = 1;
-                        if (w(ym)) d[-DP] = 1;
-                        if (w(yp)) d[DP] = 1;
-                        if (w(ym2)) d[-2 * DP] = 1;
-                        if (w(yp2)) d[2 * DP] = 1;
-                        if (w(zm)) d[-DL] = 1;
-                        if (w(zp)) d[DL] = 1;
-                        if (w(zm2)) d[-2 * DL] = 1;
-                        if (w(zp2)) d[2 * DL] = 1;
+                        if (over < xm) d[-1] = 1;
+                        if (over < xp) d[1] = 1;
+                        if (over < xm2) d[-2] = 1;
+                        if (over < xp2) d[2] = 1;
+                        if (over < ym) d[-DP] = 1;
+                        if (over < yp) d[DP] = 1;
+                        if (over < ym2) d[-2 * DP] = 1;
+                        if (over < yp2) d[2 * DP] = 1;
+                        if (over < zm) d[-DL] = 1;
+                        if (over < zp) d[DL] = 1;
+                        if (over < zm2) d[-2 * DL] = 1;
+                        if (over < zp2) d[2 * DL] = 1;
                     }
                 }
             }
         }
+        i += di;
+        c += di;
+        d += di;
+        sp += di;
         // Every fourth plane the visit ends if nothing later can be due: no node that was due at its start
         // is left ahead, and the last two planes woke nothing.
         if ((p & 3) == 3) {
-            const bool ahead = ip < 0 ? canon0 != 0u : ip < BX - 1 && (canon0 >> (ip + 1)) != 0u;
+            const int ip = p + 1 - off;  // the thread's next node, canonical
+            const bool ahead = ip <= 0 ? canon0 != 0u : ip < BX && (canon0 >> ip) != 0u;
             if (!__syncthreads_or(ahead || p - woke <= 1)) break;
         } else {
             __syncthreads();
@@ -319,61 +328,50 @@ __global__ void __launch_bounds__(BY * BZ, MINB) block_kernel(Args<Real> a) {
         const int f = a.field_list[e];
         if (lane == 0) a.fields[f].state->launch_rounds = 0;
         __syncwarp();
-        flow_advance<Real, B::MW>(a, f, true, lane);
+        const int phase = *(volatile const int*)&a.fields[f].state->phase;
+        flow_advance<Real, B::MW>(a, f, 0, 0, phase, lane);
     }
     for (;;) {
         if (threadIdx.x == 0) {
             const unsigned long long ticket = atomicAdd(&a.ctl->q_head, 1ull);
-            const unsigned long long slot = ticket & a.q_mask;
+            volatile unsigned long long* const slot = &a.q_slots[ticket & a.q_mask];
+            const unsigned long long lap = lap_of(a, ticket) >> kLapShift;
             // The limit counts from the last tiles any block queued: a long wait while others work is
-            // not a failure. The poll interval grows while nothing arrives.
+            // not a failure.
             unsigned long long t0 = global_ns();
             unsigned long long seen = *(volatile unsigned long long*)&a.ctl->q_tail;
-            unsigned nap = 16;
-            int state = 0;  // 1: the item is there; 2: leave
-            while (!state) {
-                if (*(volatile unsigned long long*)&a.q_seq[slot] == ticket + 1) {
-                    state = 1;
-                    break;
+            unsigned long long item = 0;
+            for (unsigned polls = 1;; polls++) {
+                item = *slot;
+                if (item >> kLapShift == lap) break;
+                item = 0;
+                if (*(volatile int*)&a.ctl->done || *(volatile int*)&a.ctl->abort) break;
+                if ((polls & 15u) == 0) {
+                    const unsigned long long now_p = *(volatile unsigned long long*)&a.ctl->q_tail;
+                    if (now_p != seen) {
+                        seen = now_p;
+                        t0 = global_ns();
+                    }
+                    if ((long long)(global_ns() - t0) > a.barrier_timeout_ns) {
+                        atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
+                        atomicExch(&a.ctl->abort, 1);
+                        break;
+                    }
                 }
-                if (*(volatile int*)&a.ctl->done || *(volatile int*)&a.ctl->abort) {
-                    state = 2;
-                    break;
-                }
-                const unsigned long long now_p = *(volatile unsigned long long*)&a.ctl->q_tail;
-                if (now_p != seen) {
-                    seen = now_p;
-                    t0 = global_ns();
-                }
-                if ((long long)(global_ns() - t0) > a.barrier_timeout_ns) {
-                    atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
-                    atomicExch(&a.ctl->abort, 1);
-                    state = 2;
-                    break;
-                }
-                __nanosleep(nap);
-                nap = nap < 512 ? nap * 2 : nap;
+                __nanosleep(polls < 8 ? 32 : 128);
             }
-            if (state == 1) {
+            if (item) {
+                *slot = 0ull;  // free
                 __threadfence();
-                sh->entry = __ldcg(&a.q_items[slot]);
-                __threadfence();
-                *(volatile unsigned long long*)&a.q_seq[slot] = ticket + a.q_mask + 1;  // slot free
             }
-            sh->state = state;
+            sh->entry = item;
         }
         __syncthreads();
-        if (sh->state == 2) break;
-        const unsigned long long e = sh->entry;
-        const int ff = int(e >> 32);
-        const FieldDesc<Real>& fd = a.fields[ff];
-        const GridDesc& g = a.grids[fd.grid];
-        volatile FieldState* st = fd.state;
-        const int dir = st->dir;
-        const bool second = st->phase == 1;
-        const int sx = int(e & 1023u), sy = int((e >> 10) & 1023u), sz = int((e >> 20) & 1023u);
-        if (VARZ_ANY && g.varz) my_updates += visit_block<Real, BX, BY, BZ, true>(a, g, fd, sx, sy, sz, dir, second, smem, sh, parity);
-        else my_updates += visit_block<Real, BX, BY, BZ, false>(a, g, fd, sx, sy, sz, dir, second, smem, sh, parity);
+        if (sh->entry == 0ull) break;
+        const TileItem it(sh->entry);
+        const FieldDesc<Real>& fd = a.fields[it.field];
+        if (VARZ_ANY && fd.g.varz) my_updates += visit_block<Real, BX, BY, BZ, true>(a, fd, it, smem, sh, parity);
+        else my_updates += visit_block<Real, BX, BY, BZ, false>(a, fd, it, smem, sh, parity);
         my_visits += 1;
         parity ^= 1u;
         __syncthreads();
@@ -382,12 +380,15 @@ __global__ void __launch_bounds__(BY * BZ, MINB) block_kernel(Args<Real> a) {
             int left = 0;
             if (lane == 0) {
                 __threadfence();
-                left = atomicSub((int*)&st->pending, 1) - 1;
+                left = atomicSub(&fd.state->pending, 1) - 1;
             }
             left = __shfl_sync(0xffffffffu, left, 0);
             if (left == 0) {
                 __threadfence();
-                flow_advance<Real, B::MW>(a, ff, false, lane);
+                const GridDesc& g = fd.g;
+                const int q = ((it.dir & 1) ? g.tx - 1 - it.tx : it.tx) + ((it.dir & 2) ? g.ty - 1 - it.ty : it.ty) +
+                              ((it.dir & 4) ? g.tz - 1 - it.tz : it.tz);
+                flow_advance<Real, B::MW>(a, it.field, it.dir, q + 1, it.phase, lane);
             }
         }
     }

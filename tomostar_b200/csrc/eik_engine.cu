@@ -25,9 +25,9 @@ bool tile_known(int id) { return id >= 0 && id <= kTileLastId; }
 // The shape for a job whose caller has chosen none. A deep tile crosses a diagonal in fewer steps, a flat
 // one leaves room for three blocks on an SM. With no more deep tiles in flight than two per SM (counted as
 // tiles over diagonals, summed over the fields) the steps decide: 25 fields of 81×81×41 (135 tiles) take
-// 25 ms deep and 30 flat, 10 fields of 161×161×81 (189) 119 and 138, 100 of 61×61×31 (267) 19.6 and 19.2;
-// with more, the blocks do: 50 fields of 121×121×61 (457) take 83 ms deep and 68 flat, 24 of 401×401×121
-// (1,440) 1,105 and 749.
+// 24 ms deep and 27 flat, 10 fields of 161×161×81 (189) 117 and 123, 100 of 61×61×31 (267) the same;
+// with more, the blocks do: 6 fields of 401×401×121 (360) take 376 ms deep and 358 flat, 50 of
+// 121×121×61 (457) 81 and 60, 24 of 401×401×121 (1,440) 1,092 and 673.
 static int tile_for(const ts_ctx* ctx, const EngineJob& job) {
     double in_flight = 0;
     std::vector<double> per(job.grids.size());

@@ -127,10 +127,8 @@ struct Layout {
 struct FieldState {
     int phase, round, status, changed;
     int rounds0, rounds1;
-    // The sweep ordering and diagonal in progress, its tiles still outstanding, and
-    // the rounds run in the current launch.
-    int dir, q, pending, launch_rounds;
-    int pad[4];
+    // Tiles of the diagonal in progress still outstanding, and the rounds run in the current launch.
+    int pending, launch_rounds;
 };
 
 template <typename Real>
@@ -139,12 +137,12 @@ struct FieldDesc {
     const Real* s;        // its slowness
     uint8_t* dirty;       // one flag per tile: some node of the tile is due for an update
     uint32_t* dmask;      // per tile, one bit per node (MW words): the node is due for an update
-    int grid;             // GridDesc index
     int seed_begin;       // its seed tiles: seed_tile[seed_begin .. seed_begin + seed_count), by tile id
     int seed_count;
     int cap;              // round cap per phase
     int seed_tile_lo, seed_tile_hi;  // smallest and largest seed tile id (no search outside)
     FieldState* state;               // the field's solve state; lives with the field between launches
+    GridDesc g;                      // its grid (a copy: a visit's first loads do not wait for one another)
 };
 
 struct Control {
@@ -161,7 +159,6 @@ struct Control {
 
 template <typename Real>
 struct Args {
-    const GridDesc* grids;
     const FieldDesc<Real>* fields;
     const int* seed_tile;        // tile id of each seed tile
     const uint32_t* seed_mask;   // kMaskWords words per seed tile: the fixed nodes
@@ -172,12 +169,12 @@ struct Args {
     int max_rounds_per_launch;   // rounds this launch may run (<= 0: until every field is done)
     long long epoch_budget_ns;   // after this long, each field pauses at its next round end
     long long barrier_timeout_ns;
-    // The tile queue (a bounded multi-producer multi-consumer ring): items[slot] =
-    // field << 32 | tx | ty << 10 | tz << 20. seq[slot] starts at slot; the producer of ticket t waits
-    // for seq == t, writes, and sets t + 1; its consumer waits for t + 1, reads, and sets t + capacity.
-    unsigned long long* q_items;
-    unsigned long long* q_seq;
+    // The tile queue, a bounded multi-producer multi-consumer ring of one word per slot: 0 while free, else a
+    // tile (see TileItem) with the lap of its ticket. The producer of a ticket waits for its slot to be
+    // free, its consumer for its lap; whoever takes a tile frees the slot.
+    unsigned long long* q_slots;
     unsigned long long q_mask;
+    int q_bits;                  // log2 of the slots
     Real tol;
     Real wake_rel;               // a drop wakes the neighbours when it exceeds wake_rel × the new time
     int causal;                  // a drop to t wakes only the neighbours holding more than t

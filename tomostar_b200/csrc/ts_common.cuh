@@ -65,6 +65,14 @@ TS_HDINL float real_inf<float>() { return __builtin_huge_valf(); }
 template <>
 TS_HDINL Pair real_inf<Pair>() { return Pair(__builtin_huge_valf(), 0.0f); }
 
+// Below every time in the value type's order.
+template <typename Real>
+TS_HDINL Real minus_inf();
+template <>
+TS_HDINL double minus_inf<double>() { return -__builtin_huge_val(); }
+template <>
+TS_HDINL Pair minus_inf<Pair>() { return Pair(-__builtin_huge_valf(), 0.0f); }
+
 // The C ABI precision a field value type stands for: FP64 fields are double, FP32 fields are Pair.
 template <typename Real>
 struct PrecisionOf;
