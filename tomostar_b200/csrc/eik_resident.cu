@@ -207,6 +207,8 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     }
 
     const int planes = nx + g.ny + g.nz - 2;
+    const Real tol = a.tol, wake_rel = a.wake_rel, none = minus_inf<Real>();
+    const bool causal = a.causal != 0;
     unsigned long long evals = 0;
     int phase = 0, round = 0, rounds0 = 0, rounds1 = 0, status = kRunning;
     int base = 0;  // steps of the sweeps before this one
@@ -297,19 +299,21 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
                 const int off = has_row ? off_of(j, k) : planes;
                 const int di = mx ? -1 : 1;
                 int i = mx ? nx - 1 + off - p0 : p0 - off;  // the node of plane p0 (off the row until p = off)
-                Real s = unsigned(i) < unsigned(nx) ? ldg_r(srow + i) : Real(0);
+                // The thread's node of the plane and what lies at it move one node per plane.
+                Real* c = T + row + i;
+                uint8_t* d = due + row + i;
+                const Real* sp = srow + i;
+                Real s = unsigned(i) < unsigned(nx) ? ldg_r(sp) : Real(0);
                 if (CLUSTER) rows_sync(nt + 32);
                 for (int p = p0; p < p1; p++) {
-                    const bool on = unsigned(i) < unsigned(nx);
-                    const int c = row + i;
-                    if (on && due[c] &&
-                        !(unsigned(i - fx_lo) < unsigned(fx_len) && ((fixed[c >> 5] >> (c & 31)) & 1u))) {
-                        due[c] = 0;
+                    if (unsigned(i) < unsigned(nx) && *(volatile uint8_t*)d &&
+                        !(unsigned(i - fx_lo) < unsigned(fx_len) && ((fixed[(row + i) >> 5] >> ((row + i) & 31)) & 1u))) {
+                        *d = 0;
                         evals++;
-                        const Real cur = T[c];
-                        const Real xm = T[c - 1], xp = T[c + 1], xm2 = T[c - 2], xp2 = T[c + 2];
-                        const Real ym = T[c - X], yp = T[c + X], ym2 = T[c - 2 * X], yp2 = T[c + 2 * X];
-                        const Real zm = T[c - XY], zp = T[c + XY], zm2 = T[c - 2 * XY], zp2 = T[c + 2 * XY];
+                        const Real cur = c[0];
+                        const Real xm = c[-1], xp = c[1], xm2 = c[-2], xp2 = c[2];
+                        const Real ym = c[-X], yp = c[X], ym2 = c[-2 * X], yp2 = c[2 * X];
+                        const Real zm = c[-XY], zp = c[XY], zm2 = c[-2 * XY], zp2 = c[2 * XY];
                         Real cand;
                         if (VARZ && g.varz)
                             cand = Update<Real, VARZ>::eval(s, xm, xp, xm2, xp2, ym, yp, ym2, yp2, zm, zp, zm2, zp2, wx1,
@@ -318,27 +322,32 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
                             cand = Update<Real, false>::eval(s, xm, xp, xm2, xp2, ym, yp, ym2, yp2, zm, zp, zm2, zp2, wx1,
                                                              wx2, wy1, wy2, wz1, wz2, nullptr, phase == 1);
                         if (cand < cur) {
-                            T[c] = cand;
-                            if (counts_as_change<Real>(cur, cand, a.tol)) big = true;
-                            const bool wk = wakes<Real>(cur, cand, a.wake_rel);
-                            auto w = [&](Real v) { return wk && (!a.causal || cand < v); };
-                            // The due bytes outside the grid exist (halo) and are never looked at.
-                            if (w(xm)) due[c - 1] = 1;
-                            if (w(xp)) due[c + 1] = 1;
-                            if (w(xm2)) due[c - 2] = 1;
-                            if (w(xp2)) due[c + 2] = 1;
-                            if (w(ym)) due[c - X] = 1;
-                            if (w(yp)) due[c + X] = 1;
-                            if (w(ym2)) due[c - 2 * X] = 1;
-                            if (w(yp2)) due[c + 2 * X] = 1;
-                            if (w(zm)) due[c - XY] = 1;
-                            if (w(zp)) due[c + XY] = 1;
-                            if (w(zm2)) due[c - 2 * XY] = 1;
-                            if (w(zp2)) due[c + 2 * XY] = 1;
+                            c[0] = cand;
+                            if (counts_as_change<Real>(cur, cand, tol)) big = true;
+                            if (wakes<Real>(cur, cand, wake_rel)) {
+                                // The neighbours holding more than the new time (causal rule), or all. The due
+                                // bytes outside the grid exist (halo) and are never looked at.
+                                const Real over = causal ? cand : none;
+                                if (over < xm) d[-1] = 1;
+                                if (over < xp) d[1] = 1;
+                                if (over < xm2) d[-2] = 1;
+                                if (over < xp2) d[2] = 1;
+                                if (over < ym) d[-X] = 1;
+                                if (over < yp) d[X] = 1;
+                                if (over < ym2) d[-2 * X] = 1;
+                                if (over < yp2) d[2 * X] = 1;
+                                if (over < zm) d[-XY] = 1;
+                                if (over < zp) d[XY] = 1;
+                                if (over < zm2) d[-2 * XY] = 1;
+                                if (over < zp2) d[2 * XY] = 1;
+                            }
                         }
                     }
                     i += di;  // the next plane's slowness is on its way while the others arrive
-                    s = unsigned(i) < unsigned(nx) ? ldg_r(srow + i) : Real(0);
+                    c += di;
+                    d += di;
+                    sp += di;
+                    s = unsigned(i) < unsigned(nx) ? ldg_r(sp) : Real(0);
                     if (CLUSTER) {
                         rows_sync(nt + 32);
                         if (tid == 0) *(volatile int*)&done_here = base + p + 1;
