@@ -18,7 +18,9 @@
 // A box waits only for the boxes before it along the sweep, plane by plane, and not for the boxes after
 // it, so the exchange costs a lag of a step or two per box and not a cluster barrier per step (measured
 // on 61×61×31: 11.3 ms with a barrier per step; 7.6 with the rows' threads sending and waiting
-// themselves; 6.2 with three warps of their own for it), and sweeps overlap where their orderings allow.
+// themselves; 5.7 with three warps of their own for it; 5.1, and 3.9 for 5.6 in fast mode, since these
+// skip the planes in which nothing near a face changed, most of them after the first sweeps), and
+// sweeps overlap where their orderings allow.
 //
 // The values are those of the tiled engine and of the reference to the bit: the same update on the
 // same inputs in a plane order (SphericalEikonal.cs:297-321), the same due rule
@@ -101,6 +103,15 @@ TS_DEVINL int local_acquire(unsigned addr) {
     asm volatile("ld.acquire.cluster.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
 }
+// The box's own step count, from its first thread (after the rows' barrier) to the couriers.
+TS_DEVINL void block_publish(int* at, int v) {
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(unsigned(__cvta_generic_to_shared(at))), "r"(v) : "memory");
+}
+TS_DEVINL int block_acquire(const int* at) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(unsigned(__cvta_generic_to_shared(at))) : "memory");
+    return v;
+}
 TS_DEVINL void rows_sync(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
 constexpr int kMaxPolls = 1 << 22;  // a wait longer than about a second gives up (TS_E_TIMEOUT)
 TS_DEVINL void cluster_arrive() {
@@ -110,9 +121,13 @@ TS_DEVINL void cluster_arrive() {
 TS_DEVINL void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 TS_HDINL size_t up16(size_t b) { return (b + 15) / 16 * 16; }
-// Shared memory of a box: times, due bytes, fixed bits.
+// Shared memory of a box: times, due bytes, fixed bits, and a byte per plane and pair of faces.
 TS_HDINL size_t box_elems(const ResGrid& g) { return size_t(g.pitch_x) * (g.yl + 4) * (g.zl + 4); }
-TS_HDINL size_t box_bytes(size_t elems) { return up16(8 * elems) + up16(elems) + up16((elems + 31) / 32 * 4); }
+TS_HDINL int box_planes(const ResGrid& g) { return g.nx + g.yl + g.zl; }
+TS_HDINL size_t box_bytes(const ResGrid& g) {
+    const size_t elems = box_elems(g);
+    return up16(8 * elems) + up16(elems) + up16((elems + 31) / 32 * 4) + up16(2 * size_t(box_planes(g)));
+}
 
 template <typename Real, bool VARZ, bool CLUSTER, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
@@ -128,6 +143,9 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     Real* T = reinterpret_cast<Real*>(smem);
     uint8_t* due = smem + up16(8 * elems);
     uint32_t* fixed = reinterpret_cast<uint32_t*>(due + up16(elems));
+    // Per plane of the box: a row near the y faces, near the z faces changed in it.
+    const int planes_max = box_planes(g);
+    uint8_t* moved = reinterpret_cast<uint8_t*>(fixed) + up16((elems + 31) / 32 * 4);
     const unsigned T_s = unsigned(__cvta_generic_to_shared(T)), due_s = unsigned(__cvta_generic_to_shared(due)),
                    flags_s = unsigned(__cvta_generic_to_shared(flags)),
                    done_s = unsigned(__cvta_generic_to_shared(done_by));
@@ -144,6 +162,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
 
     if (tid < 4) done_by[tid] = 0;
     if (tid == 0) done_here = 0;
+    for (int q = tid; q < 2 * planes_max && CLUSTER; q += blockDim.x) moved[q] = 0;
     // +inf everywhere, every node of the box due, the seeds (own and halo) in place.
     for (size_t q = tid; q < elems; q += blockDim.x) {
         T[q] = inf;
@@ -200,6 +219,10 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     const bool cz_ = courier && tid >= nt + 64;
     const int c_st = cz_ ? XY : X, c_n = cz_ ? nzl : nyl, c_m = cz_ ? nyl : nzl;
     const int c_box = (cz_ ? g.zl : g.yl) * c_st, c_rank = cz_ ? g.cy : 1;
+    uint8_t* const c_moved = moved + (cz_ ? planes_max : 0);
+    // Rows whose changes a courier has to carry.
+    const bool ye = CLUSTER && has_row && ((jl < 2 && by > 0) || (jl >= nyl - 2 && by + 1 < g.cy));
+    const bool ze = CLUSTER && has_row && ((kl < 2 && bz > 0) || (kl >= nzl - 2 && bz + 1 < g.cz));
     const bool c_on[2] = {courier && !idle && (cz_ ? bz > 0 : by > 0), courier && !idle && (cz_ ? bz + 1 < g.cz : by + 1 < g.cy)};
     if (CLUSTER) {
         cluster_arrive();  // every box is in place before a neighbour writes into it
@@ -262,36 +285,44 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
                 while (told < base + p1) {
                     int now = told, polls = 0;
                     while (now <= told && polls < kMaxPolls) {
-                        now = *(volatile int*)&done_here;
+                        now = __shfl_sync(0xffffffffu, block_acquire(&done_here), 0);  // one value for the warp
                         polls++;
                     }
                     if (polls >= kMaxPolls) {
                         dead = true;
                         break;
                     }
-                    // The nodes of the finished planes in the two rows at each face: their times, and the due
-                    // bytes of the neighbour's rows that they may have woken (set in this box's halo).
-                    for (int p = told - base; p < now - base; p++)
-                        for (int q = tid & 31; q < 4 * c_m; q += 32) {
-                            const int side = (q >> 1) & 1, r = q & 1, m = q >> 2;
-                            if (!c_on[side]) continue;
-                            const int n = side ? c_n - 1 - r : r;
-                            const int rj = cz_ ? m : n, rk = cz_ ? n : m;
-                            const int ip = p - off_of(j0 + rj, k0 + rk);
-                            if (unsigned(ip) >= unsigned(nx)) continue;
-                            const int c = (rk + 2) * XY + (rj + 2) * X + 2 + (mx ? nx - 1 - ip : ip);
-                            const int st = side ? c_st : -c_st, to = side ? rank + c_rank : rank - c_rank;
-                            const int cn = side ? c - c_box : c + c_box;
-                            remote_store(remote_addr(T_s + 8 * cn, to), T[c]);
-                            if (due[c + 2 * st]) {
-                                due[c + 2 * st] = 0;
-                                remote_store_u8(remote_addr(due_s + cn + 2 * st, to), 1);
-                            }
-                            if (r == 0 && due[c + st]) {
-                                due[c + st] = 0;
-                                remote_store_u8(remote_addr(due_s + cn + st, to), 1);
+                    // The nodes of the finished planes in the two rows at each face, where any changed: their
+                    // times, and the due bytes of the neighbour's rows that they may have woken (set in this
+                    // box's halo).
+                    for (int q0 = told - base; q0 < now - base; q0 += 32) {
+                        const int mine = q0 + (tid & 31);
+                        const bool has = mine < now - base && *(volatile uint8_t*)&c_moved[mine - p0] != 0;
+                        if (has) c_moved[mine - p0] = 0;
+                        for (unsigned todo = __ballot_sync(0xffffffffu, has); todo; todo &= todo - 1) {
+                            const int p = q0 + __ffs(todo) - 1;
+                            for (int q = tid & 31; q < 4 * c_m; q += 32) {
+                                const int side = (q >> 1) & 1, r = q & 1, m = q >> 2;
+                                if (!c_on[side]) continue;
+                                const int n = side ? c_n - 1 - r : r;
+                                const int rj = cz_ ? m : n, rk = cz_ ? n : m;
+                                const int ip = p - off_of(j0 + rj, k0 + rk);
+                                if (unsigned(ip) >= unsigned(nx)) continue;
+                                const int c = (rk + 2) * XY + (rj + 2) * X + 2 + (mx ? nx - 1 - ip : ip);
+                                const int st = side ? c_st : -c_st, to = side ? rank + c_rank : rank - c_rank;
+                                const int cn = side ? c - c_box : c + c_box;
+                                remote_store(remote_addr(T_s + 8 * cn, to), T[c]);
+                                if (due[c + 2 * st]) {
+                                    due[c + 2 * st] = 0;
+                                    remote_store_u8(remote_addr(due_s + cn + 2 * st, to), 1);
+                                }
+                                if (r == 0 && due[c + st]) {
+                                    due[c + st] = 0;
+                                    remote_store_u8(remote_addr(due_s + cn + st, to), 1);
+                                }
                             }
                         }
+                    }
                     told = now;
                     tell(told == base + p1 ? base + planes : told);
                 }
@@ -323,6 +354,8 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
                                                              wx2, wy1, wy2, wz1, wz2, nullptr, phase == 1);
                         if (cand < cur) {
                             c[0] = cand;
+                            if (CLUSTER && ye) moved[p - p0] = 1;
+                            if (CLUSTER && ze) moved[planes_max + p - p0] = 1;
                             if (counts_as_change<Real>(cur, cand, tol)) big = true;
                             if (wakes<Real>(cur, cand, wake_rel)) {
                                 // The neighbours holding more than the new time (causal rule), or all. The due
@@ -350,7 +383,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
                     s = unsigned(i) < unsigned(nx) ? ldg_r(sp) : Real(0);
                     if (CLUSTER) {
                         rows_sync(nt + 32);
-                        if (tid == 0) *(volatile int*)&done_here = base + p + 1;
+                        if (tid == 0) block_publish(&done_here, base + p + 1);
                     } else {
                         __syncthreads();
                     }
@@ -445,7 +478,7 @@ bool arrange(const host::Grid& g, int cluster, size_t smem_max, ResGrid& out) {
                 continue;
             t.pitch_x = (g.nx + 5) / 2 * 2;
             const int rows = t.yl * t.zl;
-            const size_t bytes = box_bytes(box_elems(t));
+            const size_t bytes = box_bytes(t);
             if (rows > kMaxRows || bytes > smem_max) continue;
             if (rows < best_rows || (rows == best_rows && bytes < best_bytes)) {
                 best_rows = rows;
@@ -517,7 +550,7 @@ int resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, 
         grids[q].pitch = job.pitch[q];
         grids[q].wz1 = weight_of<Real>(m.wz1, m.wz1_32);
         grids[q].wz2 = weight_of<Real>(m.wz2, m.wz2_32);
-        smem = std::max(smem, box_bytes(box_elems(grids[q])));
+        smem = std::max(smem, box_bytes(grids[q]));
         threads = std::max(threads, (grids[q].yl * grids[q].zl + 31) / 32 * 32);
         any_var |= grids[q].varz != 0;
         o_wx[q] = add(sizeof(Real) * m.wx.size());
