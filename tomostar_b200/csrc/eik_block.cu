@@ -36,7 +36,7 @@ __global__ void init_fields_kernel(const FieldDesc<Real>* __restrict__ fields, c
     const int64_t t0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t q = t0; q < n; q += stride) fd.T[q] = inf;
     int64_t nt = int64_t(g.tx) * g.ty * g.tz;
-    for (int64_t q = t0; q < nt; q += stride) fd.dirty[q] = 1;
+    for (int64_t q = t0; q < (nt + 15) / 16 * 16; q += stride) fd.dirty[q] = q < nt ? 1 : 0;
     for (int64_t q = t0; q < nt * mw; q += stride) fd.dmask[q] = 0xffffffffu;  // every node due (EikonalOpenCl.cs:411)
     if (t0 == 0) *fd.state = FieldState{};
 }
@@ -73,8 +73,8 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
 
     Arena A;
     // Grids.
-    std::vector<size_t> o_diag_off(ng), o_diag_tiles(ng), o_wx(ng), o_wy(ng), o_zc(ng);
-    std::vector<int> tx(ng), ty(ng), tz(ng), ndiag(ng);
+    std::vector<size_t> o_wx(ng), o_wy(ng), o_zc(ng);
+    std::vector<int> tx(ng), ty(ng), tz(ng);
     std::vector<GridDesc> descs(ng);
     for (int gi = 0; gi < ng; gi++) {
         const host::Grid& g = *grids[gi];
@@ -83,23 +83,6 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
         ty[gi] = (g.ny + BY - 1) / BY;
         tz[gi] = (g.nz + BZ - 1) / BZ;
         if (tx[gi] > 1024 || ty[gi] > 1024 || tz[gi] > 1024) return ctx->fail(TS_E_ARG, "grid too large for the tile table");
-        ndiag[gi] = tx[gi] + ty[gi] + tz[gi] - 2;
-        int nt = tx[gi] * ty[gi] * tz[gi];
-        o_diag_off[gi] = A.add(sizeof(int) * (ndiag[gi] + 1));
-        o_diag_tiles[gi] = A.add(sizeof(uint32_t) * nt);
-        // Canonical tiles ordered by diagonal (counting sort).
-        std::vector<int> cnt(ndiag[gi] + 1, 0);
-        for (int c = 0; c < tz[gi]; c++)
-            for (int b = 0; b < ty[gi]; b++)
-                for (int a = 0; a < tx[gi]; a++) cnt[a + b + c + 1]++;
-        for (int q = 0; q < ndiag[gi]; q++) cnt[q + 1] += cnt[q];
-        int* doff = A.at<int>(o_diag_off[gi]);
-        for (int q = 0; q <= ndiag[gi]; q++) doff[q] = cnt[q];
-        std::vector<int> pos(cnt.begin(), cnt.end() - 1);
-        uint32_t* dt = A.at<uint32_t>(o_diag_tiles[gi]);
-        for (int c = 0; c < tz[gi]; c++)
-            for (int b = 0; b < ty[gi]; b++)
-                for (int a = 0; a < tx[gi]; a++) dt[pos[a + b + c]++] = uint32_t(a) | (uint32_t(b) << 10) | (uint32_t(c) << 20);
         o_wx[gi] = A.add(sizeof(Real) * m.wx.size());
         for (size_t q = 0; q < m.wx.size(); q++) A.at<Real>(o_wx[gi])[q] = Real(weight_of<Real>(m.wx[q], m.wx32[q]));
         o_wy[gi] = A.add(sizeof(Real) * m.wy.size());
@@ -173,18 +156,11 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     const int running = int(field_list.size());
     size_t o_field_list = A.add(sizeof(int) * std::max<size_t>(1, field_list.size()));
     std::copy(field_list.begin(), field_list.end(), A.at<int>(o_field_list));
-    // The queue: room for twice the tiles all fields can have outstanding at once (each field has one
-    // diagonal in flight).
+    // The queue: room for every tile of every field (a tile is in it once at most, so that a producer never
+    // waits for a consumer).
     size_t qcap = 1024, need = 0;
-    {
-        std::vector<int> widest(ng, 0);
-        for (int gi = 0; gi < ng; gi++) {
-            const int* doff = A.at<int>(o_diag_off[gi]);
-            for (int q = 0; q < ndiag[gi]; q++) widest[gi] = std::max(widest[gi], doff[q + 1] - doff[q]);
-        }
-        for (int f : field_list) need += size_t(widest[fl[f]->grid]);
-        while (qcap < 2 * need) qcap *= 2;
-    }
+    for (int f : field_list) need += size_t(tx[fl[f]->grid]) * ty[fl[f]->grid] * tz[fl[f]->grid];
+    while (qcap < need) qcap *= 2;
     // Fields, control, state copies.
     size_t o_fields = A.add(sizeof(FieldDesc<Real>) * nf);
     size_t o_ctl = A.add(sizeof(Control));
@@ -194,15 +170,14 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     if (!D) return TS_E_NOMEM;
     auto* q_slots = static_cast<unsigned long long*>(ctx->buf("eng.q_slots", 8 * qcap));
     if (!q_slots) return TS_E_NOMEM;
+    auto* tokens = static_cast<unsigned*>(ctx->buf("eng.tokens", 4 * std::max<size_t>(1, need)));
+    if (!tokens) return TS_E_NOMEM;
     for (int gi = 0; gi < ng; gi++) {
         GridDesc gd{};
         const host::Grid& g = *grids[gi];
         gd.nx = g.nx; gd.ny = g.ny; gd.nz = g.nz;
         gd.tx = tx[gi]; gd.ty = ty[gi]; gd.tz = tz[gi];
-        gd.ndiag = ndiag[gi];
         gd.varz = g.variable ? 1 : 0;
-        gd.diag_off = reinterpret_cast<const int*>(D + o_diag_off[gi]);
-        gd.diag_tiles = reinterpret_cast<const uint32_t*>(D + o_diag_tiles[gi]);
         gd.wx = D + o_wx[gi];
         gd.wy = D + o_wy[gi];
         gd.zc = D + o_zc[gi];
@@ -218,6 +193,10 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
         fd.s = static_cast<const Real*>(ef.slowness);
         fd.dirty = ef.dirty;
         fd.dmask = ef.dmask;
+        if (ef.status == 0) {
+            fd.tokens = tokens;
+            tokens += size_t(tx[ef.grid]) * ty[ef.grid] * tz[ef.grid];
+        }
         fd.g = descs[ef.grid];
         fd.seed_begin = seed_begin[f];
         fd.seed_count = seed_count[f];
@@ -263,7 +242,7 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     int per_sm = 0;
     TS_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, B::kThreads, smem));
     if (per_sm < 1) return ctx->fail(TS_E_CUDA, "engine kernel does not fit on an SM");
-    // No more blocks than tiles can be outstanding at once.
+    // No more blocks than tiles.
     const int blocks = int(std::min<size_t>(size_t(per_sm) * ctx->sm_count, std::max<size_t>(1, need)));
     void* params[] = {&args};
     int64_t maxn = 0;

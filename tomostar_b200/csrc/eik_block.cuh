@@ -306,90 +306,54 @@ TS_DEVINL int visit_block(const Args<Real>& a, const FieldDesc<Real>& fd, const 
     return evals;
 }
 
-// A tile per block: the blocks take due tiles from the queue, and the block that finishes a field's last
-// tile of a diagonal moves the field on.
+// A tile per block: the blocks take due tiles from the queue, and a block that has finished one starts the
+// tiles that waited for it last.
 template <typename Real, int BX, int BY, int BZ, int MINB, bool VARZ_ANY>
 __global__ void __launch_bounds__(BY * BZ, MINB) block_kernel(Args<Real> a) {
     using B = BlockTile<Real, BX, BY, BZ>;
     extern __shared__ __align__(16) unsigned char smem[];
     BlockShared* sh = reinterpret_cast<BlockShared*>(smem + B::kTimeBytes + B::kDueBytes);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gwarp = blockIdx.x * (B::kThreads / 32) + warp, nwarps = gridDim.x * (B::kThreads / 32);
     unsigned long long my_updates = 0, my_visits = 0;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sh->arrived)), "r"(B::kThreads) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     unsigned parity = 0;
-    if (lane == 0) atomicCAS(&a.ctl->t_start, 0ull, global_ns());
-    __syncwarp();
-    // Every running field starts its launch at the first diagonal of a round.
-    for (int e = gwarp; e < a.n_active; e += nwarps) {
+    if (threadIdx.x == 0) atomicCAS(&a.ctl->t_start, 0ull, global_ns());
+    // The scheduler's list lies where the due bytes are during a visit (never written by bulk copies).
+    static_assert(B::kDueBytes >= 8 * kFlowList && B::kTimeBytes % 8 == 0, "room for the scheduler's list");
+    unsigned long long* const list = reinterpret_cast<unsigned long long*>(smem + B::kTimeBytes);
+    // Every running field starts its launch at the beginning of a round.
+    for (int e = blockIdx.x; e < a.n_active; e += gridDim.x) {
         const int f = a.field_list[e];
-        if (lane == 0) a.fields[f].state->launch_rounds = 0;
-        __syncwarp();
-        const int phase = *(volatile const int*)&a.fields[f].state->phase;
-        flow_advance<Real, B::MW>(a, f, 0, 0, phase, lane);
+        const FieldDesc<Real>& fd = a.fields[f];
+        const GridDesc& g = fd.g;
+        const int nt = g.tx * g.ty * g.tz;
+        for (int q = threadIdx.x; q < nt; q += B::kThreads)
+            __stcg(&fd.tokens[q], tokens_at_start(g, q % g.tx, q / g.tx % g.ty, q / (g.tx * g.ty)));
+        if (threadIdx.x == 0) fd.state->launch_rounds = 0;
+        __threadfence();
+        __syncthreads();
+        if (warp == 0) flow_run<Real, B::MW>(a, f, *(volatile const int*)&fd.state->phase, list, 0, lane);
+        __syncthreads();
     }
     for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned long long ticket = atomicAdd(&a.ctl->q_head, 1ull);
-            volatile unsigned long long* const slot = &a.q_slots[ticket & a.q_mask];
-            const unsigned long long lap = lap_of(a, ticket) >> kLapShift;
-            // The limit counts from the last tiles any block queued: a long wait while others work is
-            // not a failure.
-            unsigned long long t0 = global_ns();
-            unsigned long long seen = *(volatile unsigned long long*)&a.ctl->q_tail;
-            unsigned long long item = 0;
-            for (unsigned polls = 1;; polls++) {
-                item = *slot;
-                if (item >> kLapShift == lap) break;
-                item = 0;
-                if (*(volatile int*)&a.ctl->done || *(volatile int*)&a.ctl->abort) break;
-                if ((polls & 15u) == 0) {
-                    const unsigned long long now_p = *(volatile unsigned long long*)&a.ctl->q_tail;
-                    if (now_p != seen) {
-                        seen = now_p;
-                        t0 = global_ns();
-                    }
-                    if ((long long)(global_ns() - t0) > a.barrier_timeout_ns) {
-                        atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
-                        atomicExch(&a.ctl->abort, 1);
-                        break;
-                    }
-                }
-                __nanosleep(polls < 8 ? 32 : 128);
-            }
-            if (item) {
-                *slot = 0ull;  // free
-                __threadfence();
-            }
-            sh->entry = item;
-        }
+        if (threadIdx.x == 0) sh->entry = queue_pop(a);
         __syncthreads();
-        if (sh->entry == 0ull) break;
-        const TileItem it(sh->entry);
+        const unsigned long long item = sh->entry;
+        if (item == 0ull) break;
+        const TileItem it(item);
         const FieldDesc<Real>& fd = a.fields[it.field];
         if (VARZ_ANY && fd.g.varz) my_updates += visit_block<Real, BX, BY, BZ, true>(a, fd, it, smem, sh, parity);
         else my_updates += visit_block<Real, BX, BY, BZ, false>(a, fd, it, smem, sh, parity);
         my_visits += 1;
         parity ^= 1u;
         __syncthreads();
-        // The last tile of the field's diagonal moves the field on (the other warps wait for the next item).
-        if (warp == 0) {
-            int left = 0;
-            if (lane == 0) {
-                __threadfence();
-                left = atomicSub(&fd.state->pending, 1) - 1;
-            }
-            left = __shfl_sync(0xffffffffu, left, 0);
-            if (left == 0) {
-                __threadfence();
-                const GridDesc& g = fd.g;
-                const int q = ((it.dir & 1) ? g.tx - 1 - it.tx : it.tx) + ((it.dir & 2) ? g.ty - 1 - it.ty : it.ty) +
-                              ((it.dir & 4) ? g.tz - 1 - it.tz : it.tz);
-                flow_advance<Real, B::MW>(a, it.field, it.dir, q + 1, it.phase, lane);
-            }
+        if (warp == 0) {  // (the other warps wait for the next item)
+            if (lane == 0) list[0] = TileItem::pack(it.tx, it.ty, it.tz, it.dir, it.phase, it.field);
+            __syncwarp();
+            flow_run<Real, B::MW>(a, it.field, it.phase, list, 1, lane);
         }
     }
     for (int o = 16; o > 0; o >>= 1) my_updates += __shfl_down_sync(0xffffffffu, my_updates, o);

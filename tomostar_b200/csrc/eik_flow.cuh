@@ -6,17 +6,34 @@
 namespace ts {
 namespace eik {
 
-// ---- flow scheduler: no grid-wide barrier; each field advances on its own ----------------------
+// ---- flow scheduler: no grid-wide barrier; each tile starts when its neighbours allow -----------
 //
-// A field's sweep needs only that a tile diagonal q is done before diagonal q+1 of the same field
-// starts (the order argument of the engine); fields are independent. So each field keeps its own
-// position (ordering, diagonal) and count of outstanding tiles; its due tiles go into one global
-// queue that every block of the launch takes from. The warp that finishes a field's last tile of a
-// diagonal advances that field: it finds the next diagonal with due tiles (across sweeps and round
-// ends, which it evaluates for that field alone) and queues them. A launch ends when every field
-// has settled, been refused at the cap, been cancelled, or run its rounds for this launch. Waits
-// for a queue slot are bounded (globaltimer); a wait that runs out raises the abort flag and the
-// launch ends with TS_E_TIMEOUT.
+// A tile's sweep s reads the face neighbours before it along the sweep as that sweep left them and those
+// after it as the sweep before did, and wakes nodes of all of them; so it may start when the former have
+// finished sweep s, the latter sweep s − 1, and it itself sweep s − 1. Nothing else orders tiles: the
+// tiles of a field run as a wave, and the next sweep's wave starts behind it as soon as its own first
+// tiles are free (one axis or two keep their direction from one ordering to most of the next). Only a
+// round's end waits for the whole field.
+//
+// Each tile counts what it waits for in tokens, a half word for even and one for odd sweeps: one from
+// itself and one from each neighbour per sweep (a neighbour before it gives its token when it finishes
+// the sweep, one after it when it finishes the sweep before). Whoever gives the last one starts the tile:
+// with due nodes it goes into one global queue that every block of the launch takes from, without it is
+// finished at once and gives its own tokens. Tokens for a sweep two later cannot come before the tile has
+// finished this one, so two halves are enough. After a round the counts are those of its start.
+//
+// By diagonals (each started when the last tile of the one before was done) the blocks waited for the slowest
+// tile of each and in the short ones at a sweep's ends: 42 % of their time went into visits with 25 fields of
+// 81×81×41, 56 % with 50 of 121×121×61, 67 % with 10 of 161×161×81. Kernel time by diagonals and now: 24.1 ->
+// 17.8 ms, 56.4 -> 43.5, 114 -> 97; 16 uneven grids in FP32 57.9 -> 37.9; 24 of 401×401×121, which keep every
+// block busy either way, 696 -> 717: the fields now advance evenly, and their rounds' ends coincide.
+// What did not help there: handing a started tile to the visit that started it, a warp of its own for the
+// tokens that also takes the next tile during a visit, taking it by another warp while the tokens are given,
+// and diagonals in the rounds that begin with few due tiles.
+//
+// A launch ends when every field has settled, been refused at the cap, been cancelled, or run its rounds
+// for this launch. Waits for a queue slot are bounded (globaltimer); a wait that runs out raises the
+// abort flag and the launch ends with TS_E_TIMEOUT.
 
 // Ends a round of field f (SphericalEikonal.cs:297-323; EikonalOpenCl.cs:241-269). Whole warp.
 // Returns true when the field stops in this launch.
@@ -70,6 +87,10 @@ TS_DEVINL bool flow_round_end(const Args<Real>& a, int f, int lane, int& phase) 
     return stop;
 }
 
+// What a warp wrote or saw before is ordered before what it does after, for the whole GPU (lighter than
+// the sequentially consistent __threadfence()).
+TS_DEVINL void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // A tile in the queue: the tile's coordinates, the sweep ordering and phase it is due in, its field, and
 // the lap (1..63) of its ticket, so that a visit starts from the word alone.
 struct TileItem {
@@ -85,97 +106,209 @@ struct TileItem {
 constexpr int kMaxFields = 1 << 24, kLapShift = 58;
 template <typename Real>
 TS_DEVINL unsigned long long lap_of(const Args<Real>& a, unsigned long long ticket) {
-    return (1ull + (ticket >> a.q_bits) % 63ull) << kLapShift;
+    return (unsigned long long)(1u + unsigned(ticket >> a.q_bits) % 63u) << kLapShift;
 }
 
-// Moves field f to its next diagonal with due tiles, from diagonal q of ordering dir on, and queues those
-// tiles; or stops the field. Whole warp.
+// What a tile waits for: itself and its neighbours.
+TS_DEVINL unsigned tokens_needed(int gx, int gy, int gz, int tx, int ty, int tz) {
+    return 1u + unsigned(tx > 0) + unsigned(tx + 1 < gx) + unsigned(ty > 0) + unsigned(ty + 1 < gy) + unsigned(tz > 0) +
+           unsigned(tz + 1 < gz);
+}
+// Tokens a tile holds before a round's first sweep: its own and those of the neighbours after it.
+TS_DEVINL unsigned tokens_at_start(const GridDesc& g, int tx, int ty, int tz) {
+    return 1u + unsigned(tx + 1 < g.tx) + unsigned(ty + 1 < g.ty) + unsigned(tz + 1 < g.tz);
+}
+
+// A tile into the slot of its ticket. The queue has a slot for every tile, so that the slot is free.
+template <typename Real>
+TS_DEVINL void queue_put(const Args<Real>& a, unsigned long long ticket, unsigned long long word) {
+    unsigned long long* const slot = &a.q_slots[ticket & a.q_mask];
+    if (atomicCAS(slot, 0ull, word | lap_of(a, ticket)) == 0ull) return;
+    const unsigned long long t0 = global_ns();
+    while (atomicCAS(slot, 0ull, word | lap_of(a, ticket)) != 0ull) {  // its last tile not taken yet
+        if (*(volatile int*)&a.ctl->abort || (long long)(global_ns() - t0) > a.barrier_timeout_ns) {
+            atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
+            atomicExch(&a.ctl->abort, 1);
+            return;
+        }
+        __nanosleep(64);
+    }
+}
+
+// The next tile of the queue, its slot freed; waits for one. 0: the launch has ended or a wait ran out. One lane.
+template <typename Real>
+TS_DEVINL unsigned long long queue_pop(const Args<Real>& a) {
+    const unsigned long long ticket = atomicAdd(&a.ctl->q_head, 1ull);
+    volatile unsigned long long* const slot = &a.q_slots[ticket & a.q_mask];
+    const unsigned long long lap = lap_of(a, ticket) >> kLapShift;
+    // The limit counts from the last tiles any block queued: a long wait while others work is not a failure.
+    unsigned long long t0 = global_ns(), seen = *(volatile unsigned long long*)&a.ctl->q_tail;
+    for (unsigned polls = 1;; polls++) {
+        const unsigned long long item = *slot;
+        if (item >> kLapShift == lap) {
+            *slot = 0ull;
+            __threadfence();
+            return item;
+        }
+        if (*(volatile int*)&a.ctl->done || *(volatile int*)&a.ctl->abort) return 0;
+        if ((polls & 15u) == 0) {
+            const unsigned long long now = *(volatile unsigned long long*)&a.ctl->q_tail;
+            if (now != seen) {
+                seen = now;
+                t0 = global_ns();
+            }
+            if ((long long)(global_ns() - t0) > a.barrier_timeout_ns) {
+                atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
+                atomicExch(&a.ctl->abort, 1);
+                return 0;
+            }
+        }
+        __nanosleep(polls < 8 ? 32 : 128);
+    }
+}
+
+// The field that a warp moves on, and where a lane stands in it: eight lanes per finished tile, for its six
+// neighbours (axis, up) and itself (6).
+struct FlowField {
+    int gx, gy, gz;
+    unsigned* tokens;
+    const uint8_t* dirty;
+    int lane, sub, axis, up;
+};
+constexpr int kFlowList = 1024;
+
+// Gives the tokens of up to four finished tiles, the last of list[0..count); queues the due tiles that they
+// start and appends those without due nodes to the list, as finished. ended += tiles that finished the
+// round. False when the launch has been given up. Whole warp. A step is the latency of an atomic, a fence, a
+// load and a queue slot, some 3 µs, whatever it carries, and most carry one tile (steps of sixteen tiles cost
+// more instructions than they saved steps: 24 fields of 401×401×121 735 ms for 717).
+template <typename Real>
+TS_DEVINL bool flow_step(const Args<Real>& a, const FlowField& w, unsigned long long* list, int& count, int& ended) {
+    const int n = min(count, 4), q = w.lane >> 3;
+    count -= n;
+    unsigned long long word = 0;
+    unsigned add = 0, need = 0;
+    int at = 0, s = 0;
+    const bool self = w.sub == 6;
+    if (q < n && w.sub < 7) {
+        word = list[count + q];
+        TileItem z(word);
+        s = z.dir;
+        const int even = 16 * (s & 1), odd = 16 - even;
+        if (!self) {
+            const int d = w.up ? 1 : -1;
+            if (w.axis == 0) z.tx += d;
+            else if (w.axis == 1) z.ty += d;
+            else z.tz += d;
+            const bool on = unsigned(z.tx) < unsigned(w.gx) && unsigned(z.ty) < unsigned(w.gy) && unsigned(z.tz) < unsigned(w.gz);
+            // After the tile in sweep s: its token for s. Before it in s + 1: for s + 1.
+            if (on && w.up != ((s >> w.axis) & 1)) add += 1u << even;
+            if (on && w.up == (((s + 1) >> w.axis) & 1)) add += 1u << odd;
+            word += (unsigned long long)(long long)d << (10 * w.axis);
+        }
+        at = (z.tz * w.gy + z.ty) * w.gx + z.tx;
+        need = tokens_needed(w.gx, w.gy, w.gz, z.tx, z.ty, z.tz);
+        if (self) {
+            add = (1u << odd) - (need << even);
+            ended += s == 7;
+        }
+    }
+    const unsigned got = add ? atomicAdd(&w.tokens[at], add) + add : 0u;
+    // (a lane without a neighbour looks whether the launch has been given up)
+    if (__any_sync(0xffffffffu, w.sub == 7 && *(volatile int*)&a.ctl->abort)) return false;
+    const int even = 16 * (s & 1), odd = 16 - even;
+    const bool now = !self && (add >> even & 0xffffu) && (got >> even & 0xffffu) == need;
+    const bool next = add && (self || (add >> odd & 0xffffu)) && (got >> odd & 0xffffu) == need && s < 7;
+    const bool ready = now || next;
+    if (next) word += 1ull << 30;
+    if (!__any_sync(0xffffffffu, ready)) return true;
+    fence_gpu();
+    bool due = ready && __ldcg(&w.dirty[at]) != 0;
+    // Tiles without due nodes to the list (the queue when it is full), the others to the queue.
+    const unsigned before = (1u << w.lane) - 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, ready && !due);
+    if (ready && !due) {
+        const int at_q = count + __popc(m & before);
+        if (at_q < kFlowList) list[at_q] = word;
+        else due = true;
+    }
+    count = min(count + __popc(m), kFlowList);
+    const unsigned to_queue = __ballot_sync(0xffffffffu, due);
+    if (to_queue) {
+        unsigned long long ticket = 0;
+        if (w.lane == 0) ticket = atomicAdd(&a.ctl->q_tail, (unsigned long long)__popc(to_queue));
+        ticket = __shfl_sync(0xffffffffu, ticket, 0);
+        if (due) queue_put(a, ticket + __popc(to_queue & before), word);
+    }
+    __syncwarp();
+    return true;
+}
+
+// Goes on with field f after the tiles in list[0..count) (queue words without lap: the tile and the sweep it
+// finished; count 0: with a round): gives their tokens and those of the tiles without due nodes that start
+// and finish at once, queues the due tiles that start, and ends rounds. `list` is shared memory with room
+// for kFlowList words. Whole warp. (Not inlined: the visit keeps its registers.)
 template <typename Real, int MW>
-TS_DEVINL void flow_advance(const Args<Real>& a, int f, int dir, int q, int phase, int lane) {
+__device__ __noinline__ void flow_run(const Args<Real>& a, int f, int phase, unsigned long long* list, int count, int lane) {
     const FieldDesc<Real>& fd = a.fields[f];
-    const GridDesc& g = fd.g;
-    volatile FieldState* st = fd.state;
+    const int sub = lane & 7;
+    // (in registers: a fence drops the L1 lines)
+    const FlowField w{fd.g.tx, fd.g.ty, fd.g.tz, fd.tokens, fd.dirty, lane, sub, sub >> 1, sub & 1};
+    const int nt = w.gx * w.gy * w.gz;
+    FieldState* const st = fd.state;
+    fence_gpu();  // what the block wrote comes before the tokens (later steps: the fence of the one before)
+    bool begins = count == 0;
     for (;;) {
-        if (q >= g.ndiag) {
-            q = 0;
-            if (++dir == 8) {
-                dir = 0;
-                __threadfence();
-                const bool stopped = flow_round_end<Real, MW>(a, f, lane, phase);
-                __threadfence();
+        bool idle = false;
+        if (begins) {
+            begins = false;
+            // Nothing due anywhere: the round ends as it begins (a byte per tile, sixteen to a load; field
+            // buffers are padded to 256 bytes, and the bytes after the last tile are zero).
+            uint32_t some = 0;
+            for (int q = 16 * lane; q < nt; q += 512) {
+                const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w.dirty + q));
+                some |= v.x | v.y | v.z | v.w;
+            }
+            idle = !__any_sync(0xffffffffu, some != 0u);
+            if (!idle) {
+                if (lane == 0) *(volatile int*)&st->pending = nt;
                 __syncwarp();
-                if (stopped) {
-                    if (lane == 0) {
-                        st->pending = 0;
-                        if (atomicSub(&a.ctl->running, 1) == 1) atomicExch(&a.ctl->done, 1);
-                    }
+                fence_gpu();
+                const unsigned long long word = TileItem::pack(0, 0, 0, 0, phase, f);
+                if (__ldcg(&w.dirty[0])) {
+                    if (lane == 0) queue_put(a, atomicAdd(&a.ctl->q_tail, 1ull), word);
                     __syncwarp();
                     return;
                 }
+                if (lane == 0) list[0] = word;
+                count = 1;
+                __syncwarp();
             }
         }
-        auto tile = [&](int e, int& tx, int& ty, int& tz) {
-            const uint32_t pk = __ldg(&g.diag_tiles[e]);
-            const int ca = pk & 1023, cb = (pk >> 10) & 1023, cc = pk >> 20;
-            tx = (dir & 1) ? g.tx - 1 - ca : ca;
-            ty = (dir & 2) ? g.ty - 1 - cb : cb;
-            tz = (dir & 4) ? g.tz - 1 - cc : cc;
-        };
-        // Due tiles of diagonal q under ordering dir; none of them is visited before they are queued.
-        const int d0 = __ldg(&g.diag_off[q]), cnt = __ldg(&g.diag_off[q + 1]) - d0;
-        int due_total = 0;
-        unsigned kept = 0;  // lane c: the due tiles of the c-th 32 of the diagonal (1,024 tiles in all)
-        for (int b = 0; b < cnt; b += 32) {
-            bool due = false;
-            if (b + lane < cnt) {
-                int tx, ty, tz;
-                tile(d0 + b + lane, tx, ty, tz);
-                due = __ldcg(&fd.dirty[(tz * g.ty + ty) * g.tx + tx]) != 0;
+        int ended = 0;
+        while (count > 0)
+            if (!flow_step(a, w, list, count, ended)) return;
+        // The round's end, once every tile has finished its last sweep.
+        if (!idle) {
+            ended = __reduce_add_sync(0xffffffffu, ended);
+            if (!ended) return;
+            int left = 1;
+            if (lane == 0) {
+                fence_gpu();
+                left = atomicSub(&st->pending, ended) - ended;
             }
-            const unsigned m = __ballot_sync(0xffffffffu, due);
-            if (lane == (b >> 5)) kept = m;
-            due_total += __popc(m);
+            if (__shfl_sync(0xffffffffu, left, 0) != 0) return;
         }
-        if (due_total == 0) {
-            q++;
-            continue;
-        }
-        // The count before the tiles: a consumer may finish one at once.
-        if (lane == 0) st->pending = due_total;
+        fence_gpu();
+        const bool stopped = flow_round_end<Real, MW>(a, f, lane, phase);
+        fence_gpu();
         __syncwarp();
-        __threadfence();
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&a.ctl->q_tail, (unsigned long long)due_total);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        int written = 0;
-        for (int b = 0; b < cnt; b += 32) {
-            const unsigned have = __shfl_sync(0xffffffffu, kept, (b >> 5) & 31);
-            bool due = b < 1024 && ((have >> lane) & 1u);
-            unsigned long long item = 0;
-            if (due || (b >= 1024 && b + lane < cnt)) {
-                int tx, ty, tz;
-                tile(d0 + b + lane, tx, ty, tz);
-                if (b >= 1024) due = __ldcg(&fd.dirty[(tz * g.ty + ty) * g.tx + tx]) != 0;
-                item = TileItem::pack(tx, ty, tz, dir, phase, f);
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, due);
-            if (due) {
-                const unsigned long long ticket = base + written + __popc(m & ((1u << lane) - 1u));
-                unsigned long long* const slot = &a.q_slots[ticket & a.q_mask];
-                const unsigned long long t0 = global_ns();
-                while (atomicCAS(slot, 0ull, item | lap_of(a, ticket)) != 0ull) {  // its last tile not taken yet
-                    if (*(volatile int*)&a.ctl->abort || (long long)(global_ns() - t0) > a.barrier_timeout_ns) {
-                        atomicCAS(&a.ctl->error, 0, TS_E_TIMEOUT);
-                        atomicExch(&a.ctl->abort, 1);
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-            written += __popc(m);
+        if (stopped) {
+            if (lane == 0 && atomicSub(&a.ctl->running, 1) == 1) atomicExch(&a.ctl->done, 1);
+            __syncwarp();
+            return;
         }
-        __syncwarp();
-        return;
+        begins = true;
     }
 }
 

@@ -6,10 +6,11 @@
 // (SphericalEikonal.cs:297-321). A node's update reads its neighbours one and two steps away on
 // each axis; those on smaller p are already updated in this sweep, those on larger p are not yet.
 // Any visiting order in which every node comes after its axis neighbours of smaller p produces
-// exactly the same values. The engine cuts the grid into BX×BY×BZ tiles and visits them by tile
-// diagonals a'+b'+c' = q (all tiles of one diagonal at once: no two are face neighbours, and the
-// stencil only reaches face neighbours), and inside a tile by node planes. Every axis neighbour of
-// smaller p lies in the same tile or in a tile of smaller q, so the order is one of those orders.
+// exactly the same values. The engine cuts the grid into BX×BY×BZ tiles and visits a tile once the face
+// neighbours before it along the sweep are done (the stencil only reaches face neighbours), and inside a
+// tile goes by node planes. Every axis neighbour of smaller p lies in the same tile or in one of those,
+// so the order is one of those orders; a tile's neighbours after it have finished the sweep before, so
+// that sweeps may overlap.
 // Skipping a tile none of whose nodes has an input that moved since its last evaluation skips
 // only updates that would return the value already held, as the reference's dirty flags do
 // (EikonalOpenCl.cs:529-532, 608-622); the field is unchanged by it.
@@ -103,16 +104,12 @@ enum FieldStatus : int { kRunning = 0, kSettled = 1, kUnsettled = 2 };
 struct GridDesc {
     int nx, ny, nz;
     int tx, ty, tz;            // tile counts
-    int ndiag;                 // tile diagonals: tx + ty + tz - 2
     int varz;                  // variable vertical spacing (extension)
-    const int* diag_off;       // [ndiag + 1] offsets into diag_tiles
-    const uint32_t* diag_tiles;// canonical tile coords (a | b << 10 | c << 20), ordered by a + b + c
     const void* wx;            // Real[2 * nz * ny]: longitude-axis weights (w1, w2) per (k, j)
     const void* wy;            // Real[2 * nz]: latitude-axis weights per k
     const void* zc;            // Real[kZCoef * nz] when varz
     double wz1, wz2;           // depth-axis weights of a uniform grid
     int pitch;                 // elements per padded field row (see FieldDesc::T)
-    int pad;
 };
 
 // The engine's field layout: every (k, j) row is padded to `pitch` elements, node (i, j, k) at
@@ -127,7 +124,7 @@ struct Layout {
 struct FieldState {
     int phase, round, status, changed;
     int rounds0, rounds1;
-    // Tiles of the diagonal in progress still outstanding, and the rounds run in the current launch.
+    // Tiles that have not finished the round in progress, and the rounds run in the current launch.
     int pending, launch_rounds;
 };
 
@@ -137,6 +134,7 @@ struct FieldDesc {
     const Real* s;        // its slowness
     uint8_t* dirty;       // one flag per tile: some node of the tile is due for an update
     uint32_t* dmask;      // per tile, one bit per node (MW words): the node is due for an update
+    unsigned* tokens;     // per tile, what its next two sweeps have been given to start (flow scheduler)
     int seed_begin;       // its seed tiles: seed_tile[seed_begin .. seed_begin + seed_count), by tile id
     int seed_count;
     int cap;              // round cap per phase
