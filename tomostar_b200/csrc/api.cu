@@ -164,9 +164,7 @@ int ts_engine_set_tile(ts_ctx* ctx, int32_t precision, int32_t shape_id) {
     if (!ctx) return TS_E_ARG;
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     if (!ts::eik::tile_known(shape_id)) return ctx->fail(TS_E_ARG, "unknown tile shape");
-    if (precision == TS_PRECISION_F64) ctx->tile_f64 = shape_id;
-    else if (precision == TS_PRECISION_F32) ctx->tile_f32 = shape_id;
-    else return ctx->fail(TS_E_ARG, "precision must be 64 or 32");
+    if (precision != TS_PRECISION_F64 && precision != TS_PRECISION_F32) return ctx->fail(TS_E_ARG, "precision must be 64 or 32");
     (precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32) = true;
     return TS_OK;
 }

@@ -47,7 +47,6 @@ static int solve_multi_impl(ts_ctx* ctx, int n_grids, const ts_grid* grids, cons
     }
     job.tol = tol;
     job.wake_rel = mode == TS_MODE_FAST ? TS_WAKE_REL : 0.0;
-    job.tile = precision == TS_PRECISION_F64 ? ctx->tile_f64 : ctx->tile_f32;
     int64_t out_total = 0;
     for (int f = 0; f < n_fields; f++) {
         int gi = field_grid[f];
@@ -152,14 +151,12 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
     const auto& shapes = ts::eik::tile_shapes();
     int best = -1, best_sched = 0;
     double best_ms = INFINITY;
-    const int keep64 = ctx->tile_f64, keep32 = ctx->tile_f32, keep_sched = ctx->scheduler;
+    const int keep_sched = ctx->scheduler;
     const bool keep_graph = ctx->use_graph;
     const bool keep_c64 = ctx->chosen_f64, keep_c32 = ctx->chosen_f32;
     ctx->use_graph = false;
-    ctx->chosen_f64 = ctx->chosen_f32 = true;  // the shapes are what is timed
+    ctx->chosen_f64 = ctx->chosen_f32 = true;  // the engine is what is timed
     auto restore = [&]() {
-        ctx->tile_f64 = keep64;
-        ctx->tile_f32 = keep32;
         ctx->scheduler = keep_sched;
         ctx->use_graph = keep_graph;
         ctx->chosen_f64 = keep_c64;
@@ -168,8 +165,6 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
     // Every (shape, scheduler) pair; entry 2·q + scheduler of ms_per_shape.
     for (size_t q = 0; q < shapes.size(); q++) {
         for (int sched = 0; sched < 2; sched++) {
-            if (precision == TS_PRECISION_F64) ctx->tile_f64 = shapes[q].id;
-            else ctx->tile_f32 = shapes[q].id;
             ctx->scheduler = sched;
             double ms = INFINITY;
             for (int r = 0; r < std::max(1, repeats); r++) {
@@ -192,7 +187,6 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
         }
     }
     restore();
-    (precision == TS_PRECISION_F64 ? ctx->tile_f64 : ctx->tile_f32) = best;
     (precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32) = true;
     ctx->scheduler = best_sched;
     ctx->drop_graph();

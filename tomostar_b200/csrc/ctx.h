@@ -27,8 +27,7 @@ struct ts_ctx {
     size_t total_mem = 0;
     volatile int* cancel_host = nullptr;  // host-mapped, read by kernels between rounds
     int* cancel_dev = nullptr;
-    int tile_f64 = 0, tile_f32 = 0;       // engine tile shape per precision
-    int scheduler = 0;                    // engine scheduler: 0 lockstep diagonals, 1 flow (per field)
+    int scheduler = 0;                    // the engine has one; with 1 a server launch also ends on its time budget
     // The caller has chosen a tile shape or scheduler (ts_engine_set_tile, _set_scheduler, the autotuner).
     bool chosen_f64 = false, chosen_f32 = false;
     double epoch_budget_ms = 0;           // flow epochs: fields pause at the first round end after this

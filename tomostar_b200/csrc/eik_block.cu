@@ -354,19 +354,16 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
 template <typename Real>
 int engine_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids,
                  const std::vector<const host::Metric*>& metrics, const std::vector<EngineField*>& fields,
-                 double tol, double wake_rel, int tile, int max_rounds, ts_eik_stats* stats, cudaStream_t s) {
+                 double tol, double wake_rel, int max_rounds, ts_eik_stats* stats, cudaStream_t s) {
     if (fields.empty()) return TS_OK;
-    // Blocks per SM as their shared memory allows: one 32×16×16 tile (128 KB, 8 warps), three 32×16×8 tiles
-    // (77 KB, 4 warps each).
-    if (tile == kTileDeep)
-        return launch_epoch<Real, 16, 16, 1>(ctx, grids, metrics, fields, tol, wake_rel, max_rounds, stats, s);
-    return launch_epoch<Real, 16, 8, 3>(ctx, grids, metrics, fields, tol, wake_rel, max_rounds, stats, s);
+    // Three blocks per SM, as their shared memory allows (77 KB, 4 warps each).
+    return launch_epoch<Real, kTileY, kTileZ, 3>(ctx, grids, metrics, fields, tol, wake_rel, max_rounds, stats, s);
 }
 
 template int engine_epoch<Pair>(ts_ctx*, const std::vector<const host::Grid*>&, const std::vector<const host::Metric*>&,
-                                 const std::vector<EngineField*>&, double, double, int, int, ts_eik_stats*, cudaStream_t);
+                                 const std::vector<EngineField*>&, double, double, int, ts_eik_stats*, cudaStream_t);
 template int engine_epoch<double>(ts_ctx*, const std::vector<const host::Grid*>&, const std::vector<const host::Metric*>&,
-                                  const std::vector<EngineField*>&, double, double, int, int, ts_eik_stats*, cudaStream_t);
+                                  const std::vector<EngineField*>&, double, double, int, ts_eik_stats*, cudaStream_t);
 
 }  // namespace eik
 }  // namespace ts

@@ -13,32 +13,17 @@
 namespace ts {
 namespace eik {
 
-// The tile shapes compiled into the library; and the ids that callers may give: those of the shapes, or
-// one of earlier libraries' ids, which leave the choice to the job (tile_for).
+// The tile shape compiled into the library; and the ids that callers may give: its own, or one of earlier
+// libraries' shapes, for which it stands in. (A deeper tile of 32×16×16 nodes, one block per SM, crosses a grid
+// in fewer and longer visits. Since tiles start as their neighbours allow it is behind everywhere, kernel time
+// flat and deep: one field of 161×161×81 50.5 and 56.4 ms, 25 fields of 81×81×41 16.8 and 17.7, 10 of
+// 161×161×81 72 and 101, 50 of 121×121×61 51 and 80, 24 of 401×401×121 678 and 1,130.)
 const std::vector<TileShapeInfo>& tile_shapes() {
-    static const std::vector<TileShapeInfo> shapes = {{kTileFlat, kTileX, 16, 8}, {kTileDeep, kTileX, 16, 16}};
+    static const std::vector<TileShapeInfo> shapes = {{0, kTileX, kTileY, kTileZ}};
     return shapes;
 }
 
 bool tile_known(int id) { return id >= 0 && id <= kTileLastId; }
-
-// The shape for a job whose caller has chosen none. A deep tile crosses a diagonal in fewer steps, a flat
-// one leaves room for three blocks on an SM. With no more deep tiles in flight than two per SM (counted as
-// tiles over diagonals, summed over the fields) the steps decide: 25 fields of 81×81×41 (135 tiles) take
-// 24 ms deep and 27 flat, 10 fields of 161×161×81 (189) 117 and 123, 100 of 61×61×31 (267) the same;
-// with more, the blocks do: 6 fields of 401×401×121 (360) take 376 ms deep and 358 flat, 50 of
-// 121×121×61 (457) 81 and 60, 24 of 401×401×121 (1,440) 1,092 and 673.
-static int tile_for(const ts_ctx* ctx, const EngineJob& job) {
-    double in_flight = 0;
-    std::vector<double> per(job.grids.size());
-    for (size_t q = 0; q < per.size(); q++) {
-        const host::Grid& g = *job.grids[q];
-        const double tx = (g.nx + kTileX - 1) / kTileX, ty = (g.ny + 15) / 16, tz = (g.nz + 15) / 16;
-        per[q] = tx * ty * tz / (tx + ty + tz - 2);
-    }
-    for (auto& f : job.fields) in_flight += per[f.grid];
-    return in_flight <= 2.0 * ctx->sm_count ? kTileDeep : kTileFlat;
-}
 
 namespace {
 
@@ -129,7 +114,7 @@ int field_to_dense_f32_device(ts_ctx* ctx, const host::Grid& g, const FieldLayou
 int fields_to_dense_f32_device(ts_ctx* ctx, const EngineJob& job, int precision, float* out) {
     for (const auto& f : job.fields) {
         const host::Grid& g = *job.grids[f.grid];
-        FieldLayout L = field_layout(g, job.tile, precision);
+        FieldLayout L = field_layout(g, precision);
         int rc = field_to_dense_f32_device(ctx, g, L, f.T, precision, out, ctx->stream);
         if (rc) return rc;
         out += g.count();
@@ -137,8 +122,8 @@ int fields_to_dense_f32_device(ts_ctx* ctx, const EngineJob& job, int precision,
     return TS_OK;
 }
 
-FieldLayout field_layout(const host::Grid& g, int tile, int precision) {
-    const int bx = kTileX, by = 16, bz = tile == kTileDeep ? 16 : 8;
+FieldLayout field_layout(const host::Grid& g, int precision) {
+    const int bx = kTileX, by = kTileY, bz = kTileZ;
     const int hx = 2;  // 16 bytes of 8-byte values (a double, or the FP32 precision's float pair)
     (void)precision;
     const int tx = (g.nx + bx - 1) / bx, ty = (g.ny + by - 1) / by, tz = (g.nz + bz - 1) / bz;
@@ -179,10 +164,9 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     if (job.fields.empty()) return TS_OK;
     const int precision = precision_of<Real>();
     const bool chosen = is_f64<Real>() ? ctx->chosen_f64 : ctx->chosen_f32;
-    if (!chosen || (job.tile != kTileFlat && job.tile != kTileDeep)) job.tile = tile_for(ctx, job);
     // Every field's buffers from one pooled block of the context.
     std::vector<FieldLayout> layouts;
-    for (auto* g : job.grids) layouts.push_back(field_layout(*g, job.tile, precision));
+    for (auto* g : job.grids) layouts.push_back(field_layout(*g, precision));
     size_t total = 0;
     for (auto& f : job.fields) total += size_t(layouts[f.grid].bytes(precision));
     char* pool = static_cast<char*>(ctx->buf("eng.fields", total));
@@ -202,7 +186,7 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     // or a scheduler of the tiled engine, or wants the launch captured.
     if (!chosen && !ctx->use_graph)
         if (const int cluster = resident_cluster(ctx, job)) return resident_run<Real>(ctx, job, cluster, stats, ctx->stream);
-    return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, job.tile, 0, stats, ctx->stream);
+    return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, 0, stats, ctx->stream);
 }
 
 template <typename Real>
@@ -226,7 +210,6 @@ int engine_run_to_host(ts_ctx* ctx, EngineJob& job, void* out, int out_type, ts_
         sub.metrics = job.metrics;
         sub.tol = job.tol;
         sub.wake_rel = job.wake_rel;
-        sub.tile = job.tile;
         for (size_t f = f0; f < f1; f++) sub.fields.push_back(std::move(job.fields[f]));
         rc = engine_run<Real>(ctx, sub, stats);
         if (rc == TS_OK) {

@@ -44,7 +44,6 @@ struct EngineJob {
     std::vector<EngineField> fields;
     double tol = 1e-7;
     double wake_rel = 0;     // 0: the reference's dirty rule (bitwise); TS_WAKE_REL for TS_MODE_FAST
-    int tile = 0;            // tile shape id; engine_run sets the one it used
     // Set by the engine: the padded layout of each grid's fields.
     std::vector<int> pitch;
     int xoff = 0;
@@ -55,12 +54,11 @@ struct TileShapeInfo {
     int id, bx, by, bz;
 };
 const std::vector<TileShapeInfo>& tile_shapes();
-// Every tile has rows of 32 nodes; 16×8 rows (flat) or 16×16 (deep).
-constexpr int kTileX = 32, kTileFlat = 0, kTileDeep = 1, kTileLastId = 10;
-// Whether a caller may give this id (an id without a shape of its own leaves the choice to the job).
+constexpr int kTileX = 32, kTileY = 16, kTileZ = 8, kTileLastId = 10;
+// Whether a caller may give this id.
 bool tile_known(int id);
 
-// Layout of a field on a grid for a tile shape and precision: elements per padded row, x offset,
+// Layout of a field on a grid for a precision: elements per padded row, x offset,
 // tiles, due-mask words per tile.
 struct FieldLayout {
     int pitch, xoff, tiles, mask_words;
@@ -68,7 +66,7 @@ struct FieldLayout {
     int64_t elems() const;
     int64_t bytes(int precision) const;  // the whole allocation: time array, flags, masks, state
 };
-FieldLayout field_layout(const host::Grid& g, int tile, int precision);
+FieldLayout field_layout(const host::Grid& g, int precision);
 
 // One-shot: allocates every field's buffers from the context's pool and runs to completion.
 template <typename Real>
@@ -79,7 +77,7 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats);
 template <typename Real>
 int engine_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids,
                  const std::vector<const host::Metric*>& metrics, const std::vector<EngineField*>& fields,
-                 double tol, double wake_rel, int tile, int max_rounds, ts_eik_stats* stats, cudaStream_t s);
+                 double tol, double wake_rel, int max_rounds, ts_eik_stats* stats, cudaStream_t s);
 
 // Points a field's buffers into one device block of field_layout(...).bytes(precision) bytes.
 void engine_field_place(EngineField& f, const FieldLayout& L, int precision, void* block);

@@ -273,7 +273,6 @@ static int solve_impl(ts_ctx* ctx, const SolveIn& in, void* out, int out_type, t
         job.metrics.push_back(&m);
         job.tol = in.tol;
         job.wake_rel = in.mode == TS_MODE_FAST ? TS_WAKE_REL : 0.0;
-        job.tile = is_f64<Real>() ? ctx->tile_f64 : ctx->tile_f32;
         for (int f = 0; f < nf; f++) {
             EngineField ef;
             ef.grid = 0;

@@ -55,8 +55,7 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
         if (c == 0) return ctx->fail(TS_E_NOSEEDS, "no seed nodes for source " + std::to_string(tables[t].second));
     }
     const int precision = precision_of<Real>();
-    const int tile = is_f64<Real>() ? ctx->tile_f64 : ctx->tile_f32;
-    const size_t per_field = size_t(eik::field_layout(g, tile, precision).bytes(precision));
+    const size_t per_field = size_t(eik::field_layout(g, precision).bytes(precision));
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     cudaGetLastError();
@@ -73,7 +72,6 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
         job.metrics.push_back(&m);
         job.tol = 1e-7;  // SphericalEikonal.SettleTolerance
         job.wake_rel = mode == TS_MODE_FAST ? TS_WAKE_REL : 0.0;
-        job.tile = tile;
         for (int t = t0; t < t1; t++) {
             eik::EngineField ef;
             ef.grid = 0;

@@ -70,7 +70,6 @@ struct ts_server {
     ts_ctx* ctx = nullptr;
     int precision = TS_PRECISION_F64;
     int mode = TS_MODE_FAST;
-    int tile = 0;
     int rounds_per_epoch = 1;
     size_t budget = 0;
     size_t in_use = 0, peak_use = 0;
@@ -113,8 +112,8 @@ ts_grid coarsened(const ts_grid& g) {
 }
 
 // Device bytes a request holds while in flight: its fields' engine buffers and float32 tables.
-size_t footprint(const ts_ctx::Model& m, int tile, int precision, int n_fields) {
-    const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, tile, precision);
+size_t footprint(const ts_ctx::Model& m, int precision, int n_fields) {
+    const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, precision);
     const size_t per = (size_t(L.bytes(precision)) + 255) / 256 * 256 + (size_t(m.grid->count()) * 4 + 255) / 256 * 256;
     return per * size_t(n_fields);
 }
@@ -139,7 +138,7 @@ void admit(ts_server* sv) {
             continue;
         }
         const ts_ctx::Model& m = *it->second;
-        const size_t need = footprint(m, sv->tile, sv->precision, r->n_fields);
+        const size_t need = footprint(m, sv->precision, r->n_fields);
         if (need > sv->budget) {
             sv->pending.pop_front();
             finish(sv, r, TS_E_CAPACITY, "request needs more device memory than the whole budget");
@@ -157,7 +156,7 @@ void admit(ts_server* sv) {
         r->bytes = need;
         sv->in_use += need;
         sv->peak_use = std::max(sv->peak_use, sv->in_use);
-        const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, sv->tile, sv->precision);
+        const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, sv->precision);
         const size_t fb = (size_t(L.bytes(sv->precision)) + 255) / 256 * 256;
         char* p = static_cast<char*>(block);  // the fields' buffers, then their float32 tables
         const size_t esz = 8;  // model slowness: a double, or the FP32 precision's float pair
@@ -197,7 +196,7 @@ void complete_batch(ts_server* sv, const std::vector<ServeRequest*>& reqs, std::
     for (size_t k = 0; k < reqs.size(); k++) {
         ServeRequest* r = reqs[k];
         const ts_ctx::Model& m = *ctx->models.at(r->model_id);
-        const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, sv->tile, sv->precision);
+        const ts::eik::FieldLayout L = ts::eik::field_layout(*m.grid, sv->precision);
         bool settled = true;
         for (auto& ef : r->fields) {
             r->rounds[0] = std::max(r->rounds[0], ef.rounds[0]);
@@ -343,9 +342,9 @@ void serve_loop(ts_server* sv) {
         const auto te0 = Clock::now();
         if (!fl.empty()) {
             rc = sv->precision == TS_PRECISION_F64
-                     ? ts::eik::engine_epoch<double>(ctx, grids, metrics, fl, ts::kSettleTolerance, wake_rel, sv->tile,
+                     ? ts::eik::engine_epoch<double>(ctx, grids, metrics, fl, ts::kSettleTolerance, wake_rel,
                                                      sv->rounds_per_epoch, &st, ctx->stream)
-                     : ts::eik::engine_epoch<ts::Pair>(ctx, grids, metrics, fl, ts::kSettleTolerance, wake_rel, sv->tile,
+                     : ts::eik::engine_epoch<ts::Pair>(ctx, grids, metrics, fl, ts::kSettleTolerance, wake_rel,
                                                     sv->rounds_per_epoch, &st, ctx->stream);
         }
         const auto te1 = Clock::now();
@@ -422,7 +421,6 @@ int ts_serve_create(int32_t device, int32_t precision, int32_t mode, int32_t til
     sv->ctx = ctx;
     sv->precision = precision;
     sv->mode = mode;
-    sv->tile = tile == ts::eik::kTileDeep ? tile : ts::eik::kTileFlat;  // one layout for the server's life
     sv->budget = size_t(hbm_budget_bytes);
     sv->rounds_per_epoch = rounds_per_epoch > 0 ? rounds_per_epoch : 1;
     sv->loop = std::thread(serve_loop, sv);
