@@ -5,7 +5,8 @@
 // and a solve takes some 50 sweeps, so one field's time is the number of steps times the latency of a
 // step, whatever the GPU could do beside it. The tiled engine walks that chain tile by tile (a
 // 61×61×31 field: 16 tile diagonals of 44 steps and two grid-wide barriers each, 704 steps a sweep at
-// about 1 µs; 57 ms in all); here every plane of the grid is one step: 151 steps a sweep at 0.5–0.8 µs,
+// about 1 µs; 57 ms in all, 9.7 as it is now); here every plane of the grid is one step: 151 steps a sweep at
+// 0.4–0.7 µs,
 // each one shared-memory update per thread and a block barrier.
 //
 // Layout. The (y, z) rows of the grid are dealt as a cy × cz arrangement of boxes, one per block; a
@@ -499,19 +500,18 @@ constexpr size_t kSmemMax = 226 * 1024;
 // The rule. A solve's time here is its chain of steps whatever the cluster size, within 20 % (40×40×20,
 // one field: 5.0, 4.8, 4.0 and 4.2 ms with 2, 4, 8 and 16 blocks), so the size is the smallest that
 // holds every grid, or up to eight blocks where the fields still run in as many waves: a cluster lies in
-// one GPC, which takes 16 / C clusters. One wave takes a fifth of the tiled engine's chain (61×61×31, one
-// field: 6.2 ms against 28.6; 70×70×35: 9.8 against 38), and the engine's time grows slowly with the
-// fields (30 fields of 61×61×31: 45 ms against four waves here, 37 ms), so jobs of more than kMaxWaves
-// are the engine's.
-constexpr int kMaxWaves = 3;
-
+// one GPC, which takes 16 / C clusters. One wave takes half of the tiled engine's time (61×61×31, one
+// field: 5.1 ms against 9.7; 40×40×20, 54 fields: 6.3 against 9.1; 48×48×24, 18: 7.1 against 11.3), and the
+// engine's grows slowly with the fields, so more are the engine's (61×61×31, 18 fields: 18.5 against 15.6;
+// 70×70×35, 16: 22.8 against 18.4; 48×48×24, 54: 13.3 against 11.7), but for a few over a wave (61×61×31,
+// 9 fields: 11.5 against 15.1; 48×48×24, 36: 11.0 against 11.4). Grids that one block holds: up to two
+// waves (22×20×16, 148 fields: 2.0 against 4.0; 296: 3.7 against 4.1; 440: 5.1 against 5.2).
 int resident_cluster(ts_ctx* ctx, const EngineJob& job) {
     if (job.fields.empty()) return 0;
     const int gpcs = std::max(1, ctx->sm_count / 18);
-    auto waves = [&](int c) {
-        const int at_once = c == 1 ? ctx->sm_count : gpcs * (kMaxCluster / c);
-        return int((job.fields.size() + at_once - 1) / at_once);
-    };
+    const int nf = int(job.fields.size());
+    auto at_once = [&](int c) { return c == 1 ? ctx->sm_count : gpcs * (kMaxCluster / c); };
+    auto waves = [&](int c) { return (nf + at_once(c) - 1) / at_once(c); };
     auto fits = [&](int c) {
         for (auto* g : job.grids) {
             ResGrid t{};
@@ -521,7 +521,7 @@ int resident_cluster(ts_ctx* ctx, const EngineJob& job) {
     };
     int c = 1;
     while (c <= kMaxCluster && !fits(c)) c *= 2;
-    if (c > kMaxCluster || waves(c) > kMaxWaves) return 0;
+    if (c > kMaxCluster || nf > (c == 1 ? 2 * at_once(c) : at_once(c) + at_once(c) / 8)) return 0;
     if (c == 1) return 1;  // no exchange at all
     while (c < 8 && waves(2 * c) == waves(c)) c *= 2;
     return c;
