@@ -21,6 +21,9 @@ namespace {
 
 constexpr size_t kSlot = size_t(2) << 20;    // two per thread
 constexpr size_t kSmall = size_t(2) << 20;   // below this one plain copy is as fast
+// A context's first upload is a plain copy below this: making the streams and locking the slots takes 20 to
+// 30 ms, a plain upload of 64 MB six (a server that was given three models took 55 ms for it, 22 so).
+constexpr size_t kFirst = size_t(64) << 20;
 
 // Runs part(k, slots) for k in [0, n) on n threads (this one among them; a thread that cannot be started
 // leaves its part to this one). The first error of any part.
@@ -48,8 +51,8 @@ cudaError_t on_threads(ts_ctx* ctx, int n, char* slots, F part) {
 }
 
 // Threads for a copy of this size, their streams and slots made on first use; 1: a plain copy.
-int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, char** slots) {
-    if (bytes < kSmall) return 1;
+int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, bool to_host, char** slots) {
+    if (bytes < kSmall || (!to_host && bytes < kFirst && !ctx->copy_streams[0])) return 1;
     cudaPointerAttributes at{};
     const bool locked = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
     cudaGetLastError();
@@ -123,7 +126,7 @@ cudaError_t part_to_device(cudaStream_t s, char* dst, const char* src, size_t by
 int copy(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s, bool to_host) {
     if (bytes == 0) return TS_OK;
     char* slots = nullptr;
-    const int n = copy_threads(ctx, to_host ? dst : src, bytes, &slots);
+    const int n = copy_threads(ctx, to_host ? dst : src, bytes, to_host, &slots);
     if (n <= 1) {
         TS_CUDA_TRY(ctx, cudaMemcpyAsync(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, s));
         TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
