@@ -365,7 +365,7 @@ def inversion_job(device: int, threads: int) -> dict:
             tables_s = rk.last_stats.device_ms / 1e3
             out[f"fp{prec}"] = {
                 "fields_per_s": 50 / (dev / 1e3), "ms_per_50_fields": dev, "node_updates": upd,
-                "autotuned": {"shape": shape, "scheduler": ["lockstep", "flow"][sched]},
+                "autotuned": {"shape": shape, "scheduler": sched},
                 "updates_per_s": upd / (kern / 1e3),
                 "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                              "bytes_per_update": 24},
@@ -442,7 +442,7 @@ def uneven_job(device: int, threads: int) -> dict:
             ach = upd * 24 / (k_ms / 1e3) / 1e9
             out[f"fp{prec}"] = {"fields_per_s": 200 / (ms / 1e3), "ms_per_job": ms, "node_updates": int(upd),
                                 "updates_per_s": upd / (ms / 1e3), "graph_replays": int(replays),
-                                "autotuned": {"shape": shape, "scheduler": ["lockstep", "flow"][sched]},
+                                "autotuned": {"shape": shape, "scheduler": sched},
                                 "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                                              "frac": ach / peak, "bytes_per_update": 24}}
         lib.ts_engine_set_tile(s.handle, 64, 0)
@@ -765,7 +765,7 @@ def run_ours(args, problem_fn):
             "config": {"workload": f"regional forward step: 401x401x121 nodes at 0.25 km (19.46 M), {n_st} surface stations x P,S "
                                    f"= {2 * n_st} fields per GPU, Vp 1-D gradient + 3 ellipsoids +-8 % (seed 5)",
                        "global_fields": 2 * n_st * world, "tile": args.tile,
-                       "scheduler": {0: "lockstep diagonals", 1: "flow (per-field diagonals, tile queue)"}[args.scheduler],
+                       "scheduler": "flow (tiles started by their neighbours, tile queue)",
                        "mode": {0: "engine (bitwise with the reference)",
                                 2: "fast (a drop wakes only neighbours above the new time, and only when above "
                                    "1e-13 of it; within 1e-10 rel of bitwise)"}[args.mode],
@@ -775,7 +775,7 @@ def run_ours(args, problem_fn):
             "gpu_launches": 4 * launches,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "engine_kernel (FP64), 24 B per node update"},
+                         "kernel": "block_kernel (FP64), 24 B per node update"},
             "clocks": clk,
             "e2e": e2e,
             "cpu_baseline": cpu,
@@ -808,7 +808,7 @@ def main():
     ap.add_argument("--no-baselines", action="store_true")
     ap.add_argument("--fields", type=int, default=0, help="stations per step (default all 400; fewer = a small case)")
     ap.add_argument("--verbose", action="store_true", help="per-launch statistics on stderr")
-    ap.add_argument("--scheduler", type=int, default=0, help="0 lockstep diagonals, 1 flow (per field)")
+    ap.add_argument("--scheduler", type=int, default=0, help="the engine has one scheduler; 0 and 1 are accepted")
     ap.add_argument("--no-serving", action="store_true", help="skip the serving-load measurement")
     ap.add_argument("--no-forward", action="store_true", help="skip the forward step (tables + rays)")
     ap.add_argument("--no-forward-exact", action="store_true", help="skip the bitwise-mode forward step")
@@ -822,7 +822,7 @@ def main():
     ap.add_argument("--serve-tile", type=int, default=6)
     ap.add_argument("--serve-rounds", type=int, default=2, help="sweep rounds per serving epoch")
     ap.add_argument("--serve-epoch-ms", type=float, default=0.0,
-                    help="flow scheduler: fields pause at their next round end after this long (0: off)")
+                    help="scheduler 1: fields pause at their next round end after this long (0: off)")
     ap.add_argument("--dims", default="401,401,121",
                     help="grid of the regional job (smaller only for profiling captures; the bench line is 401,401,121)")
     args = ap.parse_args()

@@ -39,7 +39,7 @@ extern "C" {
 #define TS_PRECISION_F32 32
 
 /* Solve modes of ts_eik_solve. */
-#define TS_MODE_ENGINE 0  /* batched tiled engine: tile-wavefront sweeps, one cooperative launch */
+#define TS_MODE_ENGINE 0  /* batched engine: tile-wavefront sweeps, one launch */
 #define TS_MODE_PLAIN 1   /* the reference scheme as-is: one launch per diagonal plane, one field at a time */
 #define TS_MODE_FAST 2    /* the engine where a node wakes its neighbours only when it dropped by more than
                              TS_WAKE_REL of its time: last-digit changes are not propagated, so far fewer
@@ -152,14 +152,14 @@ int ts_eik_solve_noalloc(const ts_grid* grid, const double* slowness_dev, int32_
  * gate passes when *rel_err <= 1e-6 (SelfTestTolerance, :45); otherwise TS_E_SELFTEST. */
 int ts_cuda_selftest(ts_ctx* ctx, int32_t precision, double* rel_err, char* msg, int32_t cap);
 
-/* Engine tile shapes compiled into the library: writes up to cap (id, bx, by, bz) quadruples to
+/* Engine tile shapes compiled into the library (one): writes up to cap (id, bx, by, bz) quadruples to
  * shapes and returns how many exist. No reference counterpart (the OpenCL kernel is untiled). */
 int32_t ts_engine_shapes(int32_t* shapes, int32_t cap);
-/* Engine scheduler. Each field advances on its own through a shared tile queue; 1 also lets a server's
- * epoch end on time (ts_serve_set_epoch_ms). Both give the same fields. No reference counterpart. */
+/* Engine scheduler. There is one: tiles start as their neighbours allow, through a shared queue. 1 lets a server's
+ * epoch end on time (ts_serve_set_epoch_ms). Both values give the same fields. No reference counterpart. */
 int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler);
 /* Selects the engine's tile shape for one precision on this context (the autotuner's knob): an id of
- * ts_engine_shapes, or any id up to 10, which leaves the shape to each job. Without a call (and
+ * ts_engine_shapes, or any id up to 10, for which that shape stands in. Without a call (and
  * without ts_engine_set_scheduler) small grids are solved in the shared memory of one block cluster
  * per field instead of in tiles. Every choice gives the same fields. */
 int ts_engine_set_tile(ts_ctx* ctx, int32_t precision, int32_t shape_id);
@@ -177,7 +177,7 @@ int ts_eik_solve_multi(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
  * grids, fields and seeds on the same buffers) is solved again. No reference counterpart. */
 int ts_engine_set_graph(ts_ctx* ctx, int32_t enable);
 int32_t ts_engine_graph_replays(ts_ctx* ctx);
-/* Times every tile shape under both schedulers on a sample batch (ts_eik_solve_multi arguments, best
+/* Times every tile shape with both scheduler values on a sample batch (ts_eik_solve_multi arguments, best
  * of `repeats`), selects the fastest pair for `precision` on this context and returns it;
  * ms_per_shape[2q + s] receives shape q's time under scheduler s (up to cap entries). No reference
  * counterpart. */
@@ -232,7 +232,7 @@ typedef struct ts_serve_stats_t {
 int ts_serve_create(int32_t device, int32_t precision, int32_t mode, int32_t tile, int32_t scheduler,
                     double hbm_budget_bytes, int32_t rounds_per_epoch, ts_server** out);
 void ts_serve_destroy(ts_server* server);
-/* Flow scheduler only: an epoch ends once `ms` have passed, each field pausing at its next round
+/* Scheduler 1 only: an epoch ends once `ms` have passed, each field pausing at its next round
  * end (and at rounds_per_epoch rounds at the latest), so that fields of small grids keep the device
  * busy while larger ones finish their rounds. 0: rounds only. */
 int ts_serve_set_epoch_ms(ts_server* server, double ms);

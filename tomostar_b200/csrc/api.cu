@@ -153,7 +153,7 @@ int32_t ts_engine_shapes(int32_t* shapes, int32_t cap) {
 int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler) {
     if (!ctx) return TS_E_ARG;
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
-    if (scheduler != 0 && scheduler != 1) return ctx->fail(TS_E_ARG, "scheduler must be 0 (lockstep) or 1 (flow)");
+    if (scheduler != 0 && scheduler != 1) return ctx->fail(TS_E_ARG, "scheduler must be 0 or 1");
     ctx->scheduler = scheduler;
     ctx->chosen_f64 = ctx->chosen_f32 = true;
     ctx->drop_graph();

@@ -1,16 +1,16 @@
 // The block tile of the engine: 32×BY×BZ nodes swept by one thread block with one thread per (y, z) row.
 //
 // What bounds a sweep is the latency of its steps and the instructions of a step, not bandwidth (24 B of
-// the 8-byte values per update against some 45 B of DRAM traffic, a tenth of the copy rate). The warp-sized
+// the 8-byte values per update, 69 B of DRAM traffic, a seventh of the copy rate). The warp-sized
 // tiles this replaces (32×8×4 rows in registers, neighbours by shuffles) spent 757 warp instructions on a
 // step of up to 32 updates, of which the update is some 220, and crossed a 121×121×61 field in 34
 // diagonals of 44 steps. Here the tile and its two-node halo lie in shared memory in grid orientation, so
 // a step is 13 loads at fixed offsets from one address, the update, one store and a byte per woken node;
-// the field is crossed in 18 diagonals of 54 steps (32×16×8) or 14 of 62 (32×16×16). Measured against the
-// better of the earlier shapes (kernel time): 50 fields of 121×121×61 162 -> 60 ms, 10 of 161×161×81
-// (every drop wakes) 292 -> 117, 25 of 81×81×41 64 -> 24, 24 of 401×401×121 1,205 -> 673, 400 of
-// 101×101×61 341 -> 244. A plane with due nodes takes some 1,500 cycles, 850 of them the update's chain;
-// a visit's load, write-back and hand-over some 15,000, as much as ten planes.
+// the field is crossed in 18 diagonals of 54 steps. Measured against the better of the earlier shapes (kernel
+// time, both by diagonals; and since tiles start as their neighbours allow): 50 fields of 121×121×61 162 -> 56
+// -> 44 ms, 10 of 161×161×81 (every drop wakes) 292 -> 117 -> 72, 25 of 81×81×41 64 -> 24 -> 17, 24 of
+// 401×401×121 1,205 -> 673 -> 678, 400 of 101×101×61 341 -> 244 -> 260. A plane with due nodes takes some 1,500
+// cycles, 850 of them the update's chain; a visit's load, write-back and tokens some 20,000.
 //
 // Inside a tile the reference's plane order i'+j'+k' = p (mirrored coordinates) is kept: at step p the
 // thread of canonical row (j', k') evaluates the node i' = p − j' − k', one block barrier per step. A

@@ -5,9 +5,8 @@
 // and a solve takes some 50 sweeps, so one field's time is the number of steps times the latency of a
 // step, whatever the GPU could do beside it. The tiled engine walks that chain tile by tile (a
 // 61×61×31 field: 16 tile diagonals of 44 steps and two grid-wide barriers each, 704 steps a sweep at
-// about 1 µs; 57 ms in all, 9.7 as it is now); here every plane of the grid is one step: 151 steps a sweep at
-// 0.4–0.7 µs,
-// each one shared-memory update per thread and a block barrier.
+// about 1 µs; 57 ms in all, 9.7 as it is now); here every plane of the grid is one step: 151 steps a sweep
+// at 0.4–0.7 µs, each one shared-memory update per thread and a block barrier.
 //
 // Layout. The (y, z) rows of the grid are dealt as a cy × cz arrangement of boxes, one per block; a
 // thread owns one row along x. The block keeps its box's times with a two-node halo, one due byte per

@@ -205,8 +205,8 @@ class EikonalCuda:
 
     def autotune(self, grids, slownesses, field_grid, seed_sets, mode: int = L.MODE_FAST, repeats: int = 1,
                  precision: int | None = None):
-        """Times every compiled tile shape under both schedulers on the sample batch and keeps the
-        fastest pair; returns (best shape id, best scheduler, {(shape id, scheduler): ms})."""
+        """Times the compiled tile shapes (one) with both scheduler values on the sample batch and keeps
+        the fastest pair; returns (best shape id, best scheduler, {(shape id, scheduler): ms})."""
         lib = L.load()
         prec = self.precision if precision is None else precision
         ng = len(grids)

@@ -88,7 +88,7 @@ def run(seconds: float = 60.0, rate: float = 200.0, tile: int = 6, rounds_per_ep
         "complete_wall_s": (st["complete_ms"] - base["complete_ms"]) / 1e3,
         "node_updates": st["node_updates"] - base["node_updates"], "peak_hbm_gb": st["peak_bytes"] / 1e9,
         "budget_gb": budget_bytes / 1e9, "tile": tile, "rounds_per_epoch": rounds_per_epoch,
-        "scheduler": {0: "lockstep", 1: "flow"}[scheduler], "epoch_ms": epoch_ms,
+        "scheduler": scheduler, "epoch_ms": epoch_ms,
         "errors": sorted({res.error for res in results if res.status != L.TS_OK})[:3],
     }
 
