@@ -132,7 +132,9 @@ TS_HDINL size_t box_bytes(const ResGrid& g) {
 template <typename Real, bool VARZ, bool CLUSTER, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int flags[kMaxCluster];
+    // Every box's word at a round's end, in two turns: a block without a box waits for no neighbour, so the words
+    // of the next round may come before it has read these; the round after that waits for it.
+    __shared__ int flags[2][kMaxCluster];
     __shared__ int done_here;   // steps finished by this box
     __shared__ int done_by[4];  // steps finished by the neighbour box at y−1, y+1, z−1, z+1
     const int rank = CLUSTER ? int(cluster_rank()) : 0;
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     const int planes_max = box_planes(g);
     uint8_t* moved = reinterpret_cast<uint8_t*>(fixed) + up16((elems + 31) / 32 * 4);
     const unsigned T_s = unsigned(__cvta_generic_to_shared(T)), due_s = unsigned(__cvta_generic_to_shared(due)),
-                   flags_s = unsigned(__cvta_generic_to_shared(flags)),
+                   flags_s = unsigned(__cvta_generic_to_shared(&flags[0][0])),
                    done_s = unsigned(__cvta_generic_to_shared(done_by));
     const int by = rank % g.cy, bz = rank / g.cy;
     const bool idle = bz >= g.cz;  // a block the arrangement has no box for
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
     unsigned long long evals = 0;
     int phase = 0, round = 0, rounds0 = 0, rounds1 = 0, status = kRunning;
     int base = 0;  // steps of the sweeps before this one
+    int turn = 0;  // of the flags
     bool cancelled = false, dead = false;
     while (status == kRunning) {
         bool big = false;
@@ -397,11 +400,12 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(ResArgs<Real> a) {
         int mine = (tid == 0 && rank == 0 && a.cancel && *a.cancel) ? 2 : 0;
         mine = (__syncthreads_or(big) ? 1 : 0) | (__syncthreads_or(mine) ? 2 : 0) | (__syncthreads_or(dead) ? 4 : 0);
         if (CLUSTER) {
-            if (tid < a.cluster) remote_store_s32(remote_addr(flags_s + 4 * rank, tid), mine);
+            if (tid < a.cluster) remote_store_s32(remote_addr(flags_s + 4 * (turn * kMaxCluster + rank), tid), mine);
             cluster_arrive();
             cluster_wait();
             mine = 0;
-            for (int q = 0; q < a.cluster; q++) mine |= flags[q];
+            for (int q = 0; q < a.cluster; q++) mine |= flags[turn][q];
+            turn ^= 1;
         }
         if (mine & 4) {
             dead = true;
