@@ -219,7 +219,8 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     std::memcpy(image, A.h.data(), A.h.size());
     *ctl_h = Control{};
 
-    Args<Real> args{};
+    Args<Real> args;
+    std::memset(static_cast<void*>(&args), 0, sizeof args);  // its bytes are part of a captured job's signature
     args.fields = reinterpret_cast<const FieldDesc<Real>*>(D + o_fields);
     args.seed_tile = reinterpret_cast<const int*>(D + o_seed_tile);
     args.seed_mask = reinterpret_cast<const uint32_t*>(D + o_seed_mask);
@@ -281,15 +282,20 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
     };
     bool graphed = false;
     if (ctx->use_graph && max_rounds <= 0) {
-        // The job's signature: its arena bytes and the device buffers the work touches.
+        // The job's signature: its arena bytes, the buffers the work touches and what the captured launches
+        // were given by value (the kernel's arguments: the settle tolerance and the mode's wake rule among them).
         unsigned long long sig = 1469598103934665603ULL;
         auto mix = [&](const void* p, size_t n) {
             const uint8_t* b = static_cast<const uint8_t*>(p);
             for (size_t q = 0; q < n; q++) sig = (sig ^ b[q]) * 1099511628211ULL;
         };
         mix(A.h.data(), A.h.size());
-        uintptr_t ptrs[4] = {uintptr_t(D), uintptr_t(q_slots), uintptr_t(image), uintptr_t(kfn)};
+        const uintptr_t ptrs[] = {uintptr_t(D), uintptr_t(q_slots), uintptr_t(image), uintptr_t(ctl_h), uintptr_t(st_h), uintptr_t(kfn)};
         mix(ptrs, sizeof ptrs);
+        const uint64_t sizes[] = {A.h.size(), o_init, init_list.size(), sc_node.size(), o_sc_node, o_states, size_t(nf), size_t(maxn),
+                                  qcap, size_t(running), size_t(blocks), size_t(smem)};
+        mix(sizes, sizeof sizes);
+        mix(&args, sizeof args);
         if (ctx->graph_exec && ctx->graph_sig == sig) {
             TS_CUDA_TRY(ctx, cudaGraphLaunch(ctx->graph_exec, s));
             ctx->graph_replays++;
