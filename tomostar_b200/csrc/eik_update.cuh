@@ -145,6 +145,11 @@ TS_DEVINL double update64(double s, double xm, double xp, double xm2, double xp2
     const Sums64 q2 = add_term(q1, w[1], t[1]);
     const Sums64 q3 = add_term(q2, w[2], t[2]);
     const double s2 = dmul(s, s);
+    // Slowness below 2^-400 s/km: squares of times that small lose digits to underflow which the root still has, so
+    // that the tests do not decide. (Above it either the times' spread or a discriminant near sw·s² is far from
+    // that. Asked of s² as a whole number: it is known before the neighbours; asked of every discriminant
+    // the chain of a node took 5 % longer.)
+    const bool scaled = __double2hiint(s2) >= 0x0df00000;  // s² >= 2^-800
     const double n2 = fmax(n[0], n[1]);  // the largest neighbour of two terms; of three: with n[2]
     // The first candidate, from the most terms, that holds (the one of one term is formed and tested). The
     // choice is made before any root, so the lanes share one square root and one quotient; a warp whose
@@ -162,7 +167,7 @@ TS_DEVINL double update64(double s, double xm, double xp, double xm2, double xp2
         swt = k3 ? swt : k2 ? q2.swt : q1.swt;
         disc = k3 ? disc : k2 ? d2 : d1;
     }
-    if (clear) {
+    if (clear && scaled) {
         const double root = ddiv(dadd(swt, __dsqrt_rn(disc < 0.0 ? 0.0 : disc)), sw);
         return !(k3 || k2) && (disc < 0.0 || root < n[0]) ? inf : root;
     }
