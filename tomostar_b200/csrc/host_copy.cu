@@ -54,9 +54,9 @@ cudaError_t on_threads(ts_ctx* ctx, int n, char* slots, F part) {
 int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, bool to_host, char** slots) {
     if (bytes < kSmall || (!to_host && bytes < kFirst && !ctx->copy_streams[0])) return 1;
     cudaPointerAttributes at{};
-    const bool locked = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    const bool known = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (locked) return 1;  // the device reads or writes it directly
+    if (known) return 1;  // page-locked, managed or device memory: the driver's own copy, no host thread may touch it
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
     const int n = int(std::min<size_t>({size_t(ts_ctx::kCopyStreams), size_t(std::max(1u, cores / 2)), bytes / (kSlot / 2)}));
     for (int k = 0; k < n; k++)
