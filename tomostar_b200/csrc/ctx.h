@@ -7,6 +7,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/tomostar_cuda.h"
@@ -31,6 +32,8 @@ struct ts_ctx {
     // The caller has chosen a tile shape or scheduler (ts_engine_set_tile, _set_scheduler, the autotuner).
     bool chosen_f64 = false, chosen_f32 = false;
     double epoch_budget_ms = 0;           // flow epochs: fields pause at the first round end after this
+    // Whether the device can place the resident solver's clusters (kernel, blocks), as it answered once.
+    std::map<std::pair<const void*, int>, bool> clusters_placed;
     // The extended domain's 1-D background for the rays' outside time (ts_set_background): node count,
     // the nodes in the "rays.background" buffer (depths, Vp, Vs).
     int bg_n = 0;

@@ -185,7 +185,8 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     // Small grids are solved in shared memory, a cluster per field, unless the caller has chosen a shape
     // or a scheduler of the tiled engine, or wants the launch captured.
     if (!chosen && !ctx->use_graph)
-        if (const int cluster = resident_cluster(ctx, job)) return resident_run<Real>(ctx, job, cluster, stats, ctx->stream);
+        if (const int cluster = resident_cluster(ctx, job))
+            if (const auto rc = resident_run<Real>(ctx, job, cluster, stats, ctx->stream)) return *rc;
     return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, 0, stats, ctx->stream);
 }
 

@@ -531,7 +531,7 @@ int resident_cluster(ts_ctx* ctx, const EngineJob& job) {
 }
 
 template <typename Real>
-int resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, cudaStream_t s) {
+std::optional<int> resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, cudaStream_t s) {
     const int nf = int(job.fields.size()), ng = int(job.grids.size());
     // One image of everything the launch reads: grids, weights, fields, seeds, control, states.
     std::vector<uint8_t> h;
@@ -614,12 +614,8 @@ int resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, 
         return cluster > 1 ? (any_var ? resident_kernel<Real, true, true, T> : resident_kernel<Real, false, true, T>)
                            : (any_var ? resident_kernel<Real, true, false, T> : resident_kernel<Real, false, false, T>);
     };
+    const int max_threads = threads <= 256 ? 352 : 512;
     auto kfn = threads <= 256 ? pick(std::integral_constant<int, 352>()) : pick(std::integral_constant<int, 512>());
-    TS_CUDA_TRY(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    if (cluster > 8) TS_CUDA_TRY(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    EventPair ev;
-    TS_CUDA_TRY(ctx, cudaMemcpyAsync(D, image, h.size(), cudaMemcpyHostToDevice, s));
-    cudaEventRecord(ev.a, s);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(nf) * cluster);
     cfg.blockDim = dim3(threads + (cluster > 1 ? 96 : 0));
@@ -632,7 +628,38 @@ int resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, 
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = cluster > 1 ? 1 : 0;
-    TS_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kfn, args));
+    // A device that cannot place such a cluster (a part of a GPU, GPCs with few SMs) leaves the job to the engine. Asked
+    // once for a kernel and size, with the most shared memory and threads that a job may want (a query takes 0.1 ms).
+    auto placed = [&] {
+        const auto key = std::make_pair(reinterpret_cast<const void*>(kfn), cluster);
+        const auto known = ctx->clusters_placed.find(key);
+        if (known != ctx->clusters_placed.end()) return known->second;
+        cudaLaunchConfig_t most = cfg;
+        most.blockDim = dim3(max_threads);
+        most.dynamicSmemBytes = kSmemMax;
+        int at_once = 0;
+        const bool yes =
+            cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)) == cudaSuccess &&
+            (cluster <= 8 || cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+            cudaOccupancyMaxActiveClusters(&at_once, kfn, &most) == cudaSuccess && at_once > 0;
+        ctx->clusters_placed[key] = yes;
+        return yes;
+    };
+    auto takes = [&] {
+        return (cluster == 1 || placed()) &&
+               cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) == cudaSuccess;
+    };
+    if (!takes()) {
+        cudaGetLastError();
+        return std::nullopt;
+    }
+    EventPair ev;
+    TS_CUDA_TRY(ctx, cudaMemcpyAsync(D, image, h.size(), cudaMemcpyHostToDevice, s));
+    cudaEventRecord(ev.a, s);
+    if (cudaLaunchKernelEx(&cfg, kfn, args) != cudaSuccess) {
+        cudaGetLastError();
+        return std::nullopt;
+    }
     cudaEventRecord(ev.b, s);
     TS_CUDA_TRY(ctx, cudaMemcpyAsync(res_h, D + o_ctl, back, cudaMemcpyDeviceToHost, s));
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
@@ -657,8 +684,8 @@ int resident_run(ts_ctx* ctx, EngineJob& job, int cluster, ts_eik_stats* stats, 
     return TS_OK;
 }
 
-template int resident_run<double>(ts_ctx*, EngineJob&, int, ts_eik_stats*, cudaStream_t);
-template int resident_run<Pair>(ts_ctx*, EngineJob&, int, ts_eik_stats*, cudaStream_t);
+template std::optional<int> resident_run<double>(ts_ctx*, EngineJob&, int, ts_eik_stats*, cudaStream_t);
+template std::optional<int> resident_run<Pair>(ts_ctx*, EngineJob&, int, ts_eik_stats*, cudaStream_t);
 
 }  // namespace eik
 }  // namespace ts
