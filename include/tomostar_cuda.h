@@ -155,13 +155,13 @@ int ts_cuda_selftest(ts_ctx* ctx, int32_t precision, double* rel_err, char* msg,
 /* Engine tile shapes compiled into the library (one): writes up to cap (id, bx, by, bz) quadruples to
  * shapes and returns how many exist. No reference counterpart (the OpenCL kernel is untiled). */
 int32_t ts_engine_shapes(int32_t* shapes, int32_t cap);
-/* Engine scheduler. There is one: tiles start as their neighbours allow, through a shared queue. 1 lets a server's
- * epoch end on time (ts_serve_set_epoch_ms). Both values give the same fields. No reference counterpart. */
+/* Which solver a context's one-shot solves take. 0 (a new context's): the one that the job's sizes suggest, the
+ * tiled engine or, for small grids, the shared memory of one block cluster per field; a tile set before is
+ * forgotten. 1: the tiled engine, for both precisions (and a server's epoch may end on time,
+ * ts_serve_set_epoch_ms). Both give the same fields. No reference counterpart. */
 int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler);
-/* Selects the engine's tile shape for one precision on this context (the autotuner's knob): an id of
- * ts_engine_shapes, or any id up to 10, for which that shape stands in. Without a call (and
- * without ts_engine_set_scheduler) small grids are solved in the shared memory of one block cluster
- * per field instead of in tiles. Every choice gives the same fields. */
+/* Chooses the tiled engine for one precision, with an id of ts_engine_shapes or any id up to 10, for which that
+ * shape stands in; ts_engine_set_scheduler(ctx, 0) takes the choice back. Every choice gives the same fields. */
 int ts_engine_set_tile(ts_ctx* ctx, int32_t precision, int32_t shape_id);
 
 /* Many fields on grids of uneven size in one engine launch (the reference batches only fields of one
@@ -177,9 +177,10 @@ int ts_eik_solve_multi(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
  * grids, fields and seeds on the same buffers) is solved again. No reference counterpart. */
 int ts_engine_set_graph(ts_ctx* ctx, int32_t enable);
 int32_t ts_engine_graph_replays(ts_ctx* ctx);
-/* Times every tile shape with both scheduler values on a sample batch (ts_eik_solve_multi arguments, best
- * of `repeats`), selects the fastest pair for `precision` on this context and returns it;
- * ms_per_shape[2q + s] receives shape q's time under scheduler s (up to cap entries). No reference
+/* Times the solver that a context takes by itself (scheduler 0) and the tiled engine (1) on a sample batch
+ * (ts_eik_solve_multi arguments, best of `repeats`; one timing where they are the same), keeps the faster for
+ * `precision` on this context and returns it as (best_tile, best_scheduler): set_tile, then set_scheduler, gives
+ * another context the same. ms_per_shape[s] receives the time under scheduler s (up to cap entries). No reference
  * counterpart. */
 int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const double* const* slowness,
                        int32_t n_fields, const int32_t* field_grid, const int32_t* seed_offsets, const int32_t* seed_index,

@@ -155,7 +155,7 @@ int ts_engine_set_scheduler(ts_ctx* ctx, int32_t scheduler) {
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     if (scheduler != 0 && scheduler != 1) return ctx->fail(TS_E_ARG, "scheduler must be 0 or 1");
     ctx->scheduler = scheduler;
-    ctx->chosen_f64 = ctx->chosen_f32 = true;
+    ctx->chosen_f64 = ctx->chosen_f32 = scheduler == 1;  // 0: the context chooses again, a tile set before is forgotten
     ctx->drop_graph();
     return TS_OK;
 }

@@ -1,5 +1,5 @@
 // Batches of fields on grids of uneven size in one engine launch, the engine's CUDA-graph switch and
-// its tile-shape autotuner. The reference batches only fields sharing one grid and one slowness
+// the autotuner. The reference batches only fields sharing one grid and one slowness
 // (EikonalOpenCl.TrySolve, Forward/EikonalOpenCl.cs:138-166); these entry points extend that batch.
 #include <algorithm>
 #include <cmath>
@@ -148,50 +148,38 @@ int ts_engine_autotune(ts_ctx* ctx, int32_t n_grids, const ts_grid* grids, const
                        int32_t* best_scheduler, double* ms_per_shape, int32_t cap) {
     if (!ctx || !best_tile) return TS_E_ARG;
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
-    const auto& shapes = ts::eik::tile_shapes();
-    int best = -1, best_sched = 0;
-    double best_ms = INFINITY;
-    const int keep_sched = ctx->scheduler;
+    // What there is to choose: the solver that the context takes by itself (scheduler 0) and the tiled engine
+    // (1). Where the context takes the engine the two are one launch, timed once.
     const bool keep_graph = ctx->use_graph;
-    const bool keep_c64 = ctx->chosen_f64, keep_c32 = ctx->chosen_f32;
+    bool& chosen = precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32;
+    const bool keep = chosen;
     ctx->use_graph = false;
-    ctx->chosen_f64 = ctx->chosen_f32 = true;  // the engine is what is timed
-    auto restore = [&]() {
-        ctx->scheduler = keep_sched;
-        ctx->use_graph = keep_graph;
-        ctx->chosen_f64 = keep_c64;
-        ctx->chosen_f32 = keep_c32;
-    };
-    // Every (shape, scheduler) pair; entry 2·q + scheduler of ms_per_shape.
-    for (size_t q = 0; q < shapes.size(); q++) {
-        for (int sched = 0; sched < 2; sched++) {
-            ctx->scheduler = sched;
-            double ms = INFINITY;
-            for (int r = 0; r < std::max(1, repeats); r++) {
-                ts_eik_stats st{};
-                int rc = ts_eik_solve_multi(ctx, n_grids, grids, slowness, n_fields, field_grid, seed_offsets,
-                                            seed_index, seed_time, precision, mode, 1e-7, 0, nullptr, TS_OUT_NONE, &st);
-                if (rc) {
-                    restore();
-                    return rc;
-                }
-                ms = std::min(ms, st.device_ms);
+    double ms[2] = {INFINITY, INFINITY};
+    bool same = false;
+    for (int sched = 0; sched < 2 && !same; sched++) {
+        chosen = sched == 1;
+        for (int r = -1; r < std::max(1, repeats); r++) {  // the first makes the buffers and does not count
+            ts_eik_stats st{};
+            int rc = ts_eik_solve_multi(ctx, n_grids, grids, slowness, n_fields, field_grid, seed_offsets, seed_index,
+                                        seed_time, precision, mode, 1e-7, 0, nullptr, TS_OUT_NONE, &st);
+            if (rc) {
+                ctx->use_graph = keep_graph;
+                chosen = keep;
+                return rc;
             }
-            const int32_t slot = int32_t(2 * q + sched);
-            if (ms_per_shape && slot < cap) ms_per_shape[slot] = ms;
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = shapes[q].id;
-                best_sched = sched;
-            }
+            if (r >= 0) ms[sched] = std::min(ms[sched], st.device_ms);
         }
+        same = sched == 0 && !ctx->resident_last;
     }
-    restore();
-    (precision == TS_PRECISION_F64 ? ctx->chosen_f64 : ctx->chosen_f32) = true;
-    ctx->scheduler = best_sched;
+    if (same) ms[1] = ms[0];
+    ctx->use_graph = keep_graph;
+    const int best = ms[1] < ms[0] ? 1 : 0;
+    chosen = best == 1;
+    ctx->scheduler = best;
     ctx->drop_graph();
-    *best_tile = best;
-    if (best_scheduler) *best_scheduler = best_sched;
+    for (int q = 0; q < 2 && ms_per_shape && q < cap; q++) ms_per_shape[q] = ms[q];
+    *best_tile = ts::eik::tile_shapes()[0].id;
+    if (best_scheduler) *best_scheduler = best;
     return TS_OK;
 }
 

@@ -29,8 +29,10 @@ struct ts_ctx {
     volatile int* cancel_host = nullptr;  // host-mapped, read by kernels between rounds
     int* cancel_dev = nullptr;
     int scheduler = 0;                    // the engine has one; with 1 a server launch also ends on its time budget
-    // The caller has chosen a tile shape or scheduler (ts_engine_set_tile, _set_scheduler, the autotuner).
+    // The tiled engine has been chosen for a precision (ts_engine_set_tile, _set_scheduler(1), the autotuner);
+    // otherwise each job goes to the solver that its sizes suggest.
     bool chosen_f64 = false, chosen_f32 = false;
+    bool resident_last = false;           // the last one-shot job went to the resident solver
     double epoch_budget_ms = 0;           // flow epochs: fields pause at the first round end after this
     // Whether the device can place the resident solver's clusters (kernel, blocks), as it answered once.
     std::map<std::pair<const void*, int>, bool> clusters_placed;

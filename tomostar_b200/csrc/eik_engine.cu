@@ -182,11 +182,15 @@ int engine_run(ts_ctx* ctx, EngineJob& job, ts_eik_stats* stats) {
     job.pitch.clear();
     for (auto& L : layouts) job.pitch.push_back(L.pitch);
     job.xoff = layouts.empty() ? 0 : layouts[0].xoff;
-    // Small grids are solved in shared memory, a cluster per field, unless the caller has chosen a shape
-    // or a scheduler of the tiled engine, or wants the launch captured.
+    // Small grids are solved in shared memory, a cluster per field, unless the caller has chosen the tiled
+    // engine or wants the launch captured.
+    ctx->resident_last = false;
     if (!chosen && !ctx->use_graph)
         if (const int cluster = resident_cluster(ctx, job))
-            if (const auto rc = resident_run<Real>(ctx, job, cluster, stats, ctx->stream)) return *rc;
+            if (const auto rc = resident_run<Real>(ctx, job, cluster, stats, ctx->stream)) {
+                ctx->resident_last = true;
+                return *rc;
+            }
     return engine_epoch<Real>(ctx, job.grids, job.metrics, fl, job.tol, job.wake_rel, 0, stats, ctx->stream);
 }
 

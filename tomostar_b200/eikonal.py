@@ -205,8 +205,8 @@ class EikonalCuda:
 
     def autotune(self, grids, slownesses, field_grid, seed_sets, mode: int = L.MODE_FAST, repeats: int = 1,
                  precision: int | None = None):
-        """Times the compiled tile shapes (one) with both scheduler values on the sample batch and keeps
-        the fastest pair; returns (best shape id, best scheduler, {(shape id, scheduler): ms})."""
+        """Times the solver that the context takes by itself (scheduler 0) and the tiled engine (1) on the
+        sample batch and keeps the faster; returns (shape id, best scheduler, {(shape id, scheduler): ms})."""
         lib = L.load()
         prec = self.precision if precision is None else precision
         ng = len(grids)
