@@ -126,12 +126,8 @@ int32_t ts_eik_suggest_batch(ts_ctx* ctx, int64_t nodes, int32_t precision) {
     if (!ctx || nodes <= 0) return 0;
     const int64_t real = 8;  // a double, or the FP32 precision's float pair (EikonalOpenCl.Real)
     (void)precision;
-    size_t free_b = 0, total_b = 0;
     cudaSetDevice(ctx->device);
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
+    const size_t free_b = ctx->free_memory();
     // One field plus its tile flags per batch member; the slowness once (EikonalOpenCl.cs:124-131).
     int64_t per_field = nodes * real + nodes / 256 + 1;
     int64_t budget = int64_t(double(free_b) * 0.8) - 2 * nodes * real;

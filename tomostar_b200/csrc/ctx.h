@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <utility>
 #include <vector>
@@ -57,7 +58,8 @@ struct ts_ctx {
     template <typename T>
     cudaError_t alloc_async(T** p, size_t bytes, cudaStream_t s) {
         void** q = reinterpret_cast<void**>(p);
-        return pool ? cudaMallocFromPoolAsync(q, bytes, pool, s) : cudaMallocAsync(q, bytes, s);
+        return with_kept_memory(
+            [&] { return pool ? cudaMallocFromPoolAsync(q, bytes, pool, s) : cudaMallocAsync(q, bytes, s); });
     }
 
     struct Model;
@@ -70,6 +72,38 @@ struct ts_ctx {
     };
     std::map<std::string, Buf> bufs;
     std::map<std::string, Buf> pinned;    // grow-only pinned host buffers
+    // Buffers of finished calls that only spare the next call of their kind its allocation: given back when the
+    // device is short of memory. A call that asks for one has it to itself again.
+    std::set<std::string> kept;
+    void keep(const std::string& key) {
+        if (bufs.count(key)) kept.insert(key);
+    }
+    // An allocation; where the device has no room, once more without what only waits for later calls.
+    template <typename F>
+    cudaError_t with_kept_memory(F alloc) {
+        cudaError_t e = alloc();
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        while (!kept.empty()) release(std::string(*kept.begin()));
+        if (pool && cudaStreamSynchronize(stream) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+        return alloc();
+    }
+    cudaError_t alloc(void** p, size_t bytes) {
+        return with_kept_memory([&] { return cudaMalloc(p, bytes); });
+    }
+    // Device memory that an allocation of this context can have: free, idle in its pool, or kept.
+    size_t free_memory() {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+        uint64_t held = 0, used = 0;
+        if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+            free_b += size_t(held - used);
+        cudaGetLastError();
+        if (std::unique_lock<std::recursive_mutex> lk(mu, std::try_to_lock); lk)
+            for (const auto& key : kept) free_b += bufs[key].n;
+        return free_b;
+    }
 
     int fail(int code, const std::string& msg) {
         err = msg;
@@ -78,12 +112,13 @@ struct ts_ctx {
     // A grow-only named device buffer; nullptr (with err set) when the device is out of memory.
     void* buf(const std::string& key, size_t bytes) {
         Buf& b = bufs[key];
+        kept.erase(key);
         if (b.n >= bytes && b.p) return b.p;
         if (b.p) cudaFree(b.p);
         b.p = nullptr;
         b.n = 0;
         size_t want = bytes < 256 ? 256 : bytes;
-        if (cudaMalloc(&b.p, want) != cudaSuccess) {
+        if (alloc(&b.p, want) != cudaSuccess) {
             cudaGetLastError();
             b.p = nullptr;
             err = "device buffer '" + key + "' of " + std::to_string(want) + " bytes (too large for the device?)";
@@ -115,6 +150,7 @@ struct ts_ctx {
         graph_sig = 0;
     }
     void release(const std::string& key) {
+        kept.erase(key);
         auto it = bufs.find(key);
         if (it == bufs.end()) return;
         if (it->second.p) cudaFree(it->second.p);

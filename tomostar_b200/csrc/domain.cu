@@ -196,7 +196,7 @@ int ts_model_put_resampled(ts_ctx* ctx, const ts_grid* forward, const ts_grid* i
     const host::Grid ig(*inversion);
     const int64_t fn = m->grid->count(), in = ig.count();
     const size_t esz = 8;  // a double, or the float pair of the FP32 precision
-    if (cudaMalloc(&m->slowness, size_t(fn) * n_phases * esz) != cudaSuccess) {
+    if (ctx->alloc(&m->slowness, size_t(fn) * n_phases * esz) != cudaSuccess) {
         cudaGetLastError();
         m->slowness = nullptr;
         delete m;

@@ -88,6 +88,8 @@ int fields_to_dense_host(ts_ctx* ctx, const EngineJob& job, int precision, void*
             f1++;
         }
         void* stage = ctx->buf("out.stage", bytes);
+        for (; !stage && f1 > f0 + 1; stage = ctx->buf("out.stage", bytes))  // no room: fewer fields at once
+            bytes -= size_t(job.grids[job.fields[--f1].grid]->count()) * osz;
         if (!stage) return TS_E_NOMEM;
         int rc = precision == TS_PRECISION_F64
                      ? fields_to_dense_device<double>(ctx, job, f0, f1, stage, out_type, ctx->stream)
@@ -97,6 +99,7 @@ int fields_to_dense_host(ts_ctx* ctx, const EngineJob& job, int precision, void*
         dst += bytes;
         f0 = f1;
     }
+    ctx->keep("out.stage");
     return TS_OK;
 }
 

@@ -167,7 +167,7 @@ int model_put(ts_ctx* ctx, const ts_grid* grid, const double* slowness, int n_ph
     m->n_phases = n_phases;
     const size_t count = size_t(m->grid->count()) * n_phases;
     const size_t esz = 8;  // a double, or the FP32 precision's float pair (hi = the float slowness)
-    if (cudaMalloc(&m->slowness, count * esz) != cudaSuccess) {
+    if (ctx->alloc(&m->slowness, count * esz) != cudaSuccess) {
         cudaGetLastError();
         m->slowness = nullptr;
         delete m;

@@ -56,10 +56,8 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
     }
     const int precision = precision_of<Real>();
     const size_t per_field = size_t(eik::field_layout(g, precision).bytes(precision));
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    cudaGetLastError();
-    free_b += ctx->bufs.count("eng.fields") ? ctx->bufs["eng.fields"].n : 0;  // reused by the batches
+    ctx->keep("eng.fields");  // an earlier call's, reused by the batches
+    const size_t free_b = ctx->free_memory();
     const size_t room = free_b > (size_t(4) << 30) ? free_b - (size_t(4) << 30) : free_b / 2;
     const int batch = int(std::max<size_t>(1, std::min<size_t>(size_t(std::max(1, nt)), room / per_field)));
     const int cap = std::max(32, (g.nx + g.ny + g.nz) / 4);
@@ -117,9 +115,10 @@ int solve_tables(ts_ctx* ctx, const host::Grid& g, const double* slowness, int n
     }
     ctx->stats = std::to_string(r0) + "+" + std::to_string(r1) + " rounds of 8 sweeps";
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    // Small field buffers stay for the next call (mapping and unmapping 4 GB takes 5 ms, on a device in use
+    // Small field buffers are kept for the next call (mapping and unmapping 4 GB takes 5 ms, on a device in use
     // up to hundreds); large ones make room for the rows.
     if (ctx->bufs["eng.fields"].n > ctx->total_mem / 8) ctx->release("eng.fields");
+    else ctx->keep("eng.fields");
     return TS_OK;
 }
 
@@ -166,7 +165,7 @@ static int forward_impl(ts_ctx* ctx, const ts_grid* fwd_def, const double* slown
     if (rc) return rc;
     const std::string table_stats = ctx->stats;
     const auto t_tables = std::chrono::steady_clock::now();
-    // Arrivals → rays (the engine's field buffers were released for the rows).
+    // Arrivals → rays (the engine's field buffers are released or kept, which leaves them to the rows).
     std::vector<int32_t> table_of(std::max(1, n_arr));
     std::vector<double> ev(3 * std::max(1, n_arr));
     for (int a = 0; a < n_arr; a++) {

@@ -405,12 +405,10 @@ int ts_lsqr_solve_rows(ts_ctx* ctx, ts_rows* rows, int32_t n, const double* b, d
     gather_values<<<kBlocks * 4, kThreads, 0, s>>>(nnz, d_perm, len, d_tva);
     TS_CUDA_TRY(ctx, cudaGetLastError());
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    // Scratch of small systems stays for the next one (four frees and allocations take milliseconds).
-    if (sizeof(int) * 3 * size_t(nnz) > ctx->total_mem / 32) {
-        ctx->release("lsqr.perm");
-        ctx->release("lsqr.trow");
-        ctx->release("lsqr.tsrc");
-        ctx->release("lsqr.cnt");
+    // Scratch of small systems is kept for the next one (four frees and allocations take milliseconds).
+    for (const char* key : {"lsqr.perm", "lsqr.trow", "lsqr.tsrc", "lsqr.cnt"}) {
+        if (sizeof(int) * 3 * size_t(nnz) > ctx->total_mem / 32) ctx->release(key);
+        else ctx->keep(key);
     }
     System A{m, n, nnz, rs, ci, d_trs, d_tci, nullptr, nullptr, len, d_tva};
     return run(ctx, A, b, damp, max_iterations, atol, btol, conlim, x_out, info);

@@ -642,9 +642,7 @@ static int trace_impl(ts_ctx* ctx, const host::Grid& fwd, const float* tables_de
     for (int q = 0; q < n_rays; q++) need += cap_of[q];
     int64_t budget = std::max<int64_t>(need, 1);
     if (need > (int64_t(16) << 20)) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        cudaGetLastError();
+        const size_t free_b = ctx->free_memory();
         budget = std::max<int64_t>(int64_t(kMaxCap) * 64,
                                    std::min<int64_t>(int64_t(400) << 20, int64_t(free_b / 8 / 20)));
     }
