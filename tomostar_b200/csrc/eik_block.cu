@@ -82,7 +82,8 @@ int launch_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids, const
         tx[gi] = (g.nx + BX - 1) / BX;
         ty[gi] = (g.ny + BY - 1) / BY;
         tz[gi] = (g.nz + BZ - 1) / BZ;
-        if (tx[gi] > 1024 || ty[gi] > 1024 || tz[gi] > 1024) return ctx->fail(TS_E_ARG, "grid too large for the tile table");
+        if (tx[gi] > kMaxTilesX || ty[gi] > kMaxTilesYZ || tz[gi] > kMaxTilesYZ)
+            return ctx->fail(TS_E_ARG, "grid too large for the tile table");
         o_wx[gi] = A.add(sizeof(Real) * m.wx.size());
         for (size_t q = 0; q < m.wx.size(); q++) A.at<Real>(o_wx[gi])[q] = Real(weight_of<Real>(m.wx[q], m.wx32[q]));
         o_wy[gi] = A.add(sizeof(Real) * m.wy.size());

@@ -91,22 +91,24 @@ TS_DEVINL bool flow_round_end(const Args<Real>& a, int f, int lane, int& phase) 
 // the sequentially consistent __threadfence()).
 TS_DEVINL void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// A tile in the queue: the tile's coordinates, the sweep ordering and phase it is due in, its field, and
-// the lap (1..63) of its ticket, so that a visit starts from the word alone.
+// A tile in the queue: the tile's coordinates (11, 10 and 10 bits), the sweep ordering and phase it is due in, its
+// field, and the lap (1..31) of its ticket, so that a visit starts from the word alone.
 struct TileItem {
     int tx, ty, tz, dir, phase, field;
     TS_DEVINL static unsigned long long pack(int tx, int ty, int tz, int dir, int phase, int field) {
-        return (unsigned long long)(unsigned(tx) | (unsigned(ty) << 10) | (unsigned(tz) << 20)) |
-               ((unsigned long long)(unsigned(dir) | (unsigned(phase) << 3) | (unsigned(field) << 4)) << 30);
+        return (unsigned long long)(unsigned(tx) | (unsigned(ty) << 11) | (unsigned(tz) << 21)) |
+               ((unsigned long long)(unsigned(dir) | (unsigned(phase) << 3) | (unsigned(field) << 4)) << kDirShift);
     }
     TS_DEVINL explicit TileItem(unsigned long long w)
-        : tx(int(w & 1023u)), ty(int((w >> 10) & 1023u)), tz(int((w >> 20) & 1023u)), dir(int((w >> 30) & 7u)),
-          phase(int((w >> 33) & 1u)), field(int((w >> 34) & 0xffffffu)) {}
+        : tx(int(w & 2047u)), ty(int((w >> 11) & 1023u)), tz(int((w >> 21) & 1023u)), dir(int((w >> kDirShift) & 7u)),
+          phase(int((w >> (kDirShift + 3)) & 1u)), field(int((w >> (kDirShift + 4)) & 0xffffffu)) {}
+    static constexpr int kDirShift = 31;
+    TS_DEVINL static int shift(int axis) { return axis == 0 ? 0 : 10 * axis + 1; }
 };
-constexpr int kMaxFields = 1 << 24, kLapShift = 58;
+constexpr int kMaxTilesX = 2048, kMaxTilesYZ = 1024, kMaxFields = 1 << 24, kLapShift = 59;
 template <typename Real>
 TS_DEVINL unsigned long long lap_of(const Args<Real>& a, unsigned long long ticket) {
-    return (unsigned long long)(1u + unsigned(ticket >> a.q_bits) % 63u) << kLapShift;
+    return (unsigned long long)(1u + unsigned(ticket >> a.q_bits) % 31u) << kLapShift;
 }
 
 // What a tile waits for: itself and its neighbours.
@@ -204,7 +206,7 @@ TS_DEVINL bool flow_step(const Args<Real>& a, const FlowField& w, unsigned long 
             // After the tile in sweep s: its token for s. Before it in s + 1: for s + 1.
             if (on && w.up != ((s >> w.axis) & 1)) add += 1u << even;
             if (on && w.up == (((s + 1) >> w.axis) & 1)) add += 1u << odd;
-            word += (unsigned long long)(long long)d << (10 * w.axis);
+            word += (unsigned long long)(long long)d << TileItem::shift(w.axis);
         }
         at = (z.tz * w.gy + z.ty) * w.gx + z.tx;
         need = tokens_needed(w.gx, w.gy, w.gz, z.tx, z.ty, z.tz);
@@ -220,7 +222,7 @@ TS_DEVINL bool flow_step(const Args<Real>& a, const FlowField& w, unsigned long 
     const bool now = !self && (add >> even & 0xffffu) && (got >> even & 0xffffu) == need;
     const bool next = add && (self || (add >> odd & 0xffffu)) && (got >> odd & 0xffffu) == need && s < 7;
     const bool ready = now || next;
-    if (next) word += 1ull << 30;
+    if (next) word += 1ull << TileItem::kDirShift;
     if (!__any_sync(0xffffffffu, ready)) return true;
     fence_gpu();
     bool due = ready && __ldcg(&w.dirty[at]) != 0;
