@@ -123,13 +123,13 @@ cudaError_t part_to_device(cudaStream_t s, char* dst, const char* src, size_t by
     return cudaStreamSynchronize(s);
 }
 
-int copy(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s, bool to_host) {
+int copy(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s, bool to_host, bool wait = true) {
     if (bytes == 0) return TS_OK;
     char* slots = nullptr;
     const int n = copy_threads(ctx, to_host ? dst : src, bytes, to_host, &slots);
     if (n <= 1) {
         TS_CUDA_TRY(ctx, cudaMemcpyAsync(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, s));
-        TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        if (wait) TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
         return TS_OK;
     }
     // The parts' streams follow what s has queued.
@@ -165,6 +165,10 @@ __global__ void pairs_kernel(const double* a, Pair* b, size_t n) {
 
 int copy_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
     return copy(ctx, dst, src, bytes, s, true);
+}
+
+int queue_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    return copy(ctx, dst, src, bytes, s, true, false);
 }
 
 int copy_to_device(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {

@@ -9,6 +9,10 @@ namespace ts {
 // bytes from device src, as stream s leaves it, to host dst; returns when dst holds them.
 int copy_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
 
+// The same for one of several copies: a copy that is not split over threads is only queued on s, and dst holds the
+// bytes once s has been waited for.
+int queue_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 // bytes from host src to device dst, after what stream s has queued; work queued on s afterwards sees
 // them, and src may change when the call returns.
 int copy_to_device(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);

@@ -1015,9 +1015,9 @@ int ts_rows_copy(ts_rows* rows, int32_t* row_ptr, int32_t* col, float* len, doub
     if (row_ptr) TS_CUDA_TRY(ctx, cudaMemcpyAsync(row_ptr, rows->row_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, s));
     if (tcalc_grad && n) TS_CUDA_TRY(ctx, cudaMemcpyAsync(tcalc_grad, rows->tcg, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s));
     if (col && rows->nnz)
-        if (int rc = copy_to_host(ctx, col, rows->col, sizeof(int) * size_t(rows->nnz), s)) return rc;
+        if (int rc = queue_to_host(ctx, col, rows->col, sizeof(int) * size_t(rows->nnz), s)) return rc;
     if (len && rows->nnz)
-        if (int rc = copy_to_host(ctx, len, rows->len, sizeof(float) * size_t(rows->nnz), s)) return rc;
+        if (int rc = queue_to_host(ctx, len, rows->len, sizeof(float) * size_t(rows->nnz), s)) return rc;
     if (ok && n) TS_CUDA_TRY(ctx, cudaMemcpyAsync(ok, rows->ok, size_t(n), cudaMemcpyDeviceToHost, s));
     TS_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     return TS_OK;

@@ -272,8 +272,8 @@ void complete_batch(ts_server* sv, const std::vector<ServeRequest*>& reqs, std::
         ServeRequest* r = reqs[k];
         if (codes[k] != TS_OK || !r->tables_out) continue;
         const int64_t n = ctx->models.at(r->model_id)->grid->count();
-        const int rc = ts::copy_to_host(ctx, r->tables_out, r->tables_dev, sizeof(float) * size_t(n) * r->n_fields,
-                                        ctx->stream);
+        const int rc = ts::queue_to_host(ctx, r->tables_out, r->tables_dev, sizeof(float) * size_t(n) * r->n_fields,
+                                         ctx->stream);
         if (rc) fail(k, rc);
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
