@@ -1,5 +1,5 @@
 """Results into memory whose pages are there, not there and partly there, around the sizes at which a copy is split
-over threads (2 MB) and at which it is split whatever the pages (32 MB)."""
+over threads (2 MB) and at which it is split whatever the pages (24 MB)."""
 import ctypes as C
 import mmap
 
@@ -14,7 +14,7 @@ from tomostar_b200.synthetic import regular_grid
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kb", [1900, 2049, 2600, 31 * 1024 + 900, 32 * 1024 + 4])
+@pytest.mark.parametrize("kb", [1900, 2049, 2600, 23 * 1024 + 900, 24 * 1024 + 4])
 def test_pages(kb):
     g = regular_grid(4, 4, 16, 1.0)  # tables of 1 kB
     tabs = np.random.default_rng(kb).random((kb, g.count), np.float32)

@@ -7,6 +7,7 @@
 
 #include "ctx.h"
 #include "eik_engine.h"
+#include "host_copy.h"
 #include "host_geo.h"
 
 using ts::host::Grid;
@@ -101,6 +102,7 @@ void ts_cuda_destroy(ts_ctx* ctx) {
         if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
         for (cudaStream_t s : ctx->copy_streams)
             if (s) cudaStreamDestroy(s);
+        ts::free_copy_slots(ctx);
         cudaStreamDestroy(ctx->stream);
         // Allocations still held (rows not yet freed) keep the pool's memory until they are freed.
         if (ctx->pool) cudaMemPoolDestroy(ctx->pool);

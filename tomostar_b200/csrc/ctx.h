@@ -21,6 +21,7 @@ struct ts_ctx {
     // Streams of the threads of a pageable copy (host_copy.cu; created on use).
     static constexpr int kCopyStreams = 8;
     cudaStream_t copy_streams[kCopyStreams] = {};
+    void* copy_slots = nullptr;  // page-locked, two per stream
     std::recursive_mutex mu;  // calls on one context are serialised (EikonalOpenCl.cs:64,165)
     std::string err;
     std::string stats;

@@ -23,9 +23,10 @@ namespace ts {
 namespace {
 
 constexpr size_t kSlot = size_t(2) << 20;    // two per thread
+constexpr size_t kSlotBytes = size_t(ts_ctx::kCopyStreams) * 2 * kSlot;
 constexpr size_t kSmall = size_t(2) << 20;   // below this one plain copy is as fast
-// A context's first upload is a plain copy below this: making the streams and locking the slots takes 20 to
-// 30 ms, a plain upload of 64 MB six (a server that was given three models took 55 ms for it, 22 so).
+// An upload below this is a plain copy until another copy has made the streams: making them and locking the
+// slots takes seven to ten ms once, a plain upload of 64 MB six.
 constexpr size_t kFirst = size_t(64) << 20;
 
 // Runs part(k, slots) for k in [0, n) on n threads (this one among them; a thread that cannot be started
@@ -54,10 +55,10 @@ cudaError_t on_threads(ts_ctx* ctx, int n, char* slots, F part) {
 }
 
 // Whether the pages of host memory are there (a sample of them): into memory touched before, one plain copy to
-// the host is faster below 32 MB, where starting the threads takes longer than they save (2.5 MB 0.17 ms plain and
-// 0.50 by threads, 8 MB 0.45 and 0.74, 24 MB 1.40 and 1.48, 32 MB 1.87 and 1.56); into new memory the threads share
-// its page faults (2.5 MB 1.30 and 0.92, 8 MB 4.1 and 1.7).
-constexpr size_t kTouched = size_t(32) << 20;
+// the host is faster below 24 MB, where starting the threads takes longer than they save (2.5 MB 0.17 ms plain and
+// 0.50 by threads, 8 MB 0.45 and 0.74, 24 MB 1.40 and 1.48, 32 MB 1.87 and 1.56); into new memory the threads
+// share its page faults (2.5 MB 1.30 and 0.92, 8 MB 4.1 and 1.7).
+constexpr size_t kTouched = size_t(24) << 20;
 bool touched(const void* p, size_t bytes) {
     const size_t page = size_t(sysconf(_SC_PAGESIZE));
     for (int k = 0; k < 8; k++) {
@@ -68,14 +69,32 @@ bool touched(const void* p, size_t bytes) {
     return true;
 }
 
+// The threads' page-locked slots, made on first use; null where they cannot be had. Locking 32 MB in huge pages
+// takes 5 ms, touching them included; cudaHostAlloc took 15 to 17 for it.
+char* page_locked_slots(ts_ctx* ctx) {
+    if (ctx->copy_slots) return static_cast<char*>(ctx->copy_slots);
+    void* p = mmap(nullptr, kSlotBytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) return nullptr;
+    madvise(p, kSlotBytes, MADV_HUGEPAGE);  // (a wish: small pages do as well)
+    std::memset(p, 0, kSlotBytes);
+    if (cudaHostRegister(p, kSlotBytes, cudaHostRegisterDefault) != cudaSuccess) {
+        cudaGetLastError();
+        munmap(p, kSlotBytes);
+        return nullptr;
+    }
+    ctx->copy_slots = p;
+    return static_cast<char*>(p);
+}
+
 // Threads for a copy of this size, their streams and slots made on first use; 1: a plain copy.
 int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, bool to_host, char** slots) {
-    if (bytes < kSmall || (!to_host && bytes < kFirst && !ctx->copy_streams[0])) return 1;
+    if (bytes < kSmall) return 1;
     cudaPointerAttributes at{};
     const bool known = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (to_host && bytes < kTouched && touched(host, bytes)) return 1;
     if (known) return 1;  // page-locked, managed or device memory: the driver's own copy, no host thread may touch it
+    if (to_host && bytes < kTouched && touched(host, bytes)) return 1;
+    if (!to_host && !ctx->copy_streams[0] && bytes < kFirst) return 1;
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
     const int n = int(std::min<size_t>({size_t(ts_ctx::kCopyStreams), size_t(std::max(1u, cores / 2)), bytes / (kSlot / 2)}));
     for (int k = 0; k < n; k++)
@@ -85,8 +104,7 @@ int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, bool to_host, char
             ctx->copy_streams[k] = nullptr;
             return 1;
         }
-    *slots = static_cast<char*>(ctx->host_buf("copy.slots", size_t(ts_ctx::kCopyStreams) * 2 * kSlot));
-    if (!*slots) cudaGetLastError();
+    *slots = page_locked_slots(ctx);
     return *slots ? n : 1;
 }
 
@@ -181,6 +199,13 @@ __global__ void pairs_kernel(const double* a, Pair* b, size_t n) {
 }
 
 }  // namespace
+
+void free_copy_slots(ts_ctx* ctx) {
+    if (!ctx->copy_slots) return;
+    cudaHostUnregister(ctx->copy_slots);
+    munmap(ctx->copy_slots, kSlotBytes);
+    ctx->copy_slots = nullptr;
+}
 
 int copy_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
     return copy(ctx, dst, src, bytes, s, true);

@@ -17,6 +17,9 @@ int queue_to_host(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStr
 // them, and src may change when the call returns.
 int copy_to_device(ts_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
 
+// Gives back what the copies of a context that is being destroyed used (its streams idle).
+void free_copy_slots(ts_ctx* ctx);
+
 // count doubles of the host as FP64 values, or as the FP32 precision's float pairs (formed on the device).
 int upload_values(ts_ctx* ctx, double* dst, const double* src, size_t count, cudaStream_t s);
 int upload_values(ts_ctx* ctx, Pair* dst, const double* src, size_t count, cudaStream_t s);
