@@ -22,6 +22,7 @@ struct ts_ctx {
     static constexpr int kCopyStreams = 8;
     cudaStream_t copy_streams[kCopyStreams] = {};
     void* copy_slots = nullptr;  // page-locked, two per stream
+    size_t uploaded = 0;  // bytes that went up before there were any
     std::recursive_mutex mu;  // calls on one context are serialised (EikonalOpenCl.cs:64,165)
     std::string err;
     std::string stats;
