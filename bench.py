@@ -317,7 +317,7 @@ def _fmm_sample_fields_per_s(grids, slownesses, seed_sets, threads: int):
 def inversion_job(device: int, threads: int) -> dict:
     """The forward step of a synthetic inversion (121x121x61 at 0.5 km, 25 stations x P,S = 50 fields,
     7,500 rays) in FP64 and FP32 (the paired-float scheme): engine fields/s (the 50 fields in one
-    launch, P and S as two slowness models of the grid, the tile shape and scheduler picked by the
+    launch, P and S as two slowness models of the grid, the solver picked by the
     autotuner on the job), its roofline, the forward step through ts_forward (tables + Jacobian rows),
     the plain per-plane GPU path on one field and the CPU solver on a sample of fields."""
     from oracle import oracle as O
@@ -401,8 +401,8 @@ def inversion_job(device: int, threads: int) -> dict:
 
 def uneven_job(device: int, threads: int) -> dict:
     """200 sources each on its own grid (48-192 x 48-192 x 32-96 nodes, half with geometric depth
-    spacing) solved in one persistent engine launch, the tile shape and scheduler picked by the
-    autotuner on a 40-grid sample, the job captured as a CUDA graph and replayed; FP32 (the named
+    spacing) solved in one persistent engine launch, captured as a CUDA graph and replayed (the autotuner
+    runs on a 40-grid sample before); FP32 (the named
     precision: paired floats) and FP64. Baselines: the plain per-plane GPU path and the CPU solver on
     samples of the grids."""
     from tomostar_b200 import _lib as L
@@ -808,7 +808,7 @@ def main():
     ap.add_argument("--no-baselines", action="store_true")
     ap.add_argument("--fields", type=int, default=0, help="stations per step (default all 400; fewer = a small case)")
     ap.add_argument("--verbose", action="store_true", help="per-launch statistics on stderr")
-    ap.add_argument("--scheduler", type=int, default=0, help="the engine has one scheduler; 0 and 1 are accepted")
+    ap.add_argument("--scheduler", type=int, default=0, help="0: the solver each job's sizes suggest, 1: the tiled engine")
     ap.add_argument("--no-serving", action="store_true", help="skip the serving-load measurement")
     ap.add_argument("--no-forward", action="store_true", help="skip the forward step (tables + rays)")
     ap.add_argument("--no-forward-exact", action="store_true", help="skip the bitwise-mode forward step")

@@ -363,7 +363,8 @@ int engine_epoch(ts_ctx* ctx, const std::vector<const host::Grid*>& grids,
                  const std::vector<const host::Metric*>& metrics, const std::vector<EngineField*>& fields,
                  double tol, double wake_rel, int max_rounds, ts_eik_stats* stats, cudaStream_t s) {
     if (fields.empty()) return TS_OK;
-    // Three blocks per SM, as their shared memory allows (77 KB, 4 warps each).
+    // Three blocks per SM, as their shared memory (77 KB each) and their registers (156 to 164 a thread in FP64)
+    // allow.
     return launch_epoch<Real, kTileY, kTileZ, 3>(ctx, grids, metrics, fields, tol, wake_rel, max_rounds, stats, s);
 }
 

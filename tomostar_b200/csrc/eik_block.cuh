@@ -7,10 +7,11 @@
 // diagonals of 44 steps. Here the tile and its two-node halo lie in shared memory in grid orientation, so
 // a step is 13 loads at fixed offsets from one address, the update, one store and a byte per woken node;
 // the field is crossed in 18 diagonals of 54 steps. Measured against the better of the earlier shapes (kernel
-// time, both by diagonals; and since tiles start as their neighbours allow): 50 fields of 121×121×61 162 -> 56
-// -> 44 ms, 10 of 161×161×81 (every drop wakes) 292 -> 117 -> 72, 25 of 81×81×41 64 -> 24 -> 17, 24 of
-// 401×401×121 1,205 -> 673 -> 678, 400 of 101×101×61 341 -> 244 -> 260. A plane with due nodes takes some 1,500
-// cycles, 850 of them the update's chain; a visit's load, write-back and tokens some 20,000.
+// time, both by diagonals, in turn on one GPU): 50 fields of 121×121×61 162 -> 56 ms, 24 of 401×401×121
+// 1,205 -> 673, 400 of 101×101×61 341 -> 244. Since tiles start as their neighbours allow (eik_flow.cuh), all on
+// one GPU: 50 of 121×121×61 49 ms, 10 of 161×161×81 (every drop wakes) 82, 25 of 81×81×41 19, 24 of 401×401×121
+// 733, 16 uneven grids in FP32 27. A plane with due nodes takes some 1,500 cycles, 850 of them the update's
+// chain; a visit's load, write-back and tokens some 20,000.
 //
 // Inside a tile the reference's plane order i'+j'+k' = p (mirrored coordinates) is kept: at step p the
 // thread of canonical row (j', k') evaluates the node i' = p − j' − k', one block barrier per step. A
@@ -37,8 +38,7 @@ struct BlockTile {
     static constexpr int RY = BY + 4, RZ = BZ + 4;    // rows and levels, halo included
     static constexpr int LEVEL = RY * PITCH;
     static constexpr int kSlots = RY * RZ;            // row (j, k) is slot (k + 2)·RY + j + 2
-    // The first and the last two slots are corners, which nothing reads: they are not stored (with them
-    // two tiles of 32×16×16 would not fit on an SM).
+    // The first and the last two slots are corners, which nothing reads: they are not stored.
     static constexpr int kTimeBytes = (kSlots - 4) * PITCH * 8;
     // Due bytes: row r's node i is byte r·DP + 4 + i. The two bytes before a row's first node and the two
     // after its last (the first two of the next row's 36) are its x halo.

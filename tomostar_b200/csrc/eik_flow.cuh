@@ -23,10 +23,11 @@ namespace eik {
 // finished this one, so two halves are enough. After a round the counts are those of its start.
 //
 // By diagonals (each started when the last tile of the one before was done) the blocks waited for the slowest
-// tile of each and in the short ones at a sweep's ends: 42 % of their time went into visits with 25 fields of
-// 81×81×41, 56 % with 50 of 121×121×61, 67 % with 10 of 161×161×81. Kernel time by diagonals and now
-// (the first and third with the deeper tile of then): 24.1 -> 17.8 ms, 56.4 -> 43.5, 114 -> 97; 16 uneven grids in FP32 57.9 -> 37.9; 24 of 401×401×121, which keep every
-// block busy either way, 696 -> 717: the fields now advance evenly, and their rounds' ends coincide.
+// tile of each and in the short ones at a sweep's ends: 56 % of their time went into visits with 50 fields of
+// 121×121×61. Kernel time by diagonals and by tokens, in turn on one GPU: those 56.4 -> 43.5 ms, 16 uneven grids
+// in FP32 57.9 -> 37.9, 24 of 401×401×121, which keep every block busy either way, 696 -> 717: the fields now
+// advance evenly, and their rounds' ends coincide. (With a tile twice as deep, which has gone: 25 fields of
+// 81×81×41 24.1 -> 17.8, 10 of 161×161×81 114 -> 97.)
 // What did not help there: handing a started tile to the visit that started it, a warp of its own for the
 // tokens that also takes the next tile during a visit, taking it by another warp while the tokens are given,
 // and diagonals in the rounds that begin with few due tiles.
