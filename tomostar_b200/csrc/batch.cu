@@ -75,6 +75,8 @@ static int solve_multi_impl(ts_ctx* ctx, int n_grids, const ts_grid* grids, cons
     cudaEventCreate(&e1);
     cudaEventRecord(e0, ctx->stream);
     int rc = engine_run<Real>(ctx, job, stats);
+    const bool in_parts = rc == TS_E_NOMEM && n_fields > 1 && out_type != TS_OUT_NONE;
+    if (in_parts) rc = engine_run_in_parts<Real>(ctx, job, out, out_type, stats);
     cudaEventRecord(e1, ctx->stream);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -95,7 +97,7 @@ static int solve_multi_impl(ts_ctx* ctx, int n_grids, const ts_grid* grids, cons
     if (rc) return rc;
     for (auto& ef : job.fields)
         if (ef.status != 1) return ctx->fail(TS_E_UNSETTLED, "sweeping not settled within the round cap");
-    if (out_type == TS_OUT_NONE) return TS_OK;
+    if (out_type == TS_OUT_NONE || in_parts) return TS_OK;
     return fields_to_dense_host(ctx, job, precision, out, out_type);
 }
 

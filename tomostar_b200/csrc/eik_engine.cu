@@ -240,6 +240,37 @@ int engine_run_to_host(ts_ctx* ctx, EngineJob& job, void* out, int out_type, ts_
     return rc;
 }
 
+template <typename Real>
+int engine_run_in_parts(ts_ctx* ctx, EngineJob& job, void* out, int out_type, ts_eik_stats* stats) {
+    const size_t nf = job.fields.size(), osz = out_type == TS_OUT_F64 ? 8 : 4;
+    size_t per = (nf + 1) / 2;
+    char* dst = static_cast<char*>(out);
+    for (size_t f0 = 0; f0 < nf;) {
+        const size_t f1 = std::min(nf, f0 + per);
+        EngineJob sub;
+        sub.grids = job.grids;
+        sub.metrics = job.metrics;
+        sub.tol = job.tol;
+        sub.wake_rel = job.wake_rel;
+        for (size_t f = f0; f < f1; f++) sub.fields.push_back(std::move(job.fields[f]));
+        int rc = engine_run<Real>(ctx, sub, stats);
+        bool settled = true;
+        for (const auto& ef : sub.fields) settled = settled && ef.status == 1;
+        if (rc == TS_OK && settled) rc = fields_to_dense_host(ctx, sub, precision_of<Real>(), dst, out_type);
+        for (size_t f = f0; f < f1; f++) job.fields[f] = std::move(sub.fields[f - f0]);
+        if (rc == TS_E_NOMEM && per > 1) {
+            per = (per + 1) / 2;
+            continue;
+        }
+        if (rc || !settled) return rc;  // the caller looks at the fields
+        for (size_t f = f0; f < f1; f++) dst += size_t(job.grids[job.fields[f].grid]->count()) * osz;
+        f0 = f1;
+    }
+    return TS_OK;
+}
+
+template int engine_run_in_parts<double>(ts_ctx*, EngineJob&, void*, int, ts_eik_stats*);
+template int engine_run_in_parts<Pair>(ts_ctx*, EngineJob&, void*, int, ts_eik_stats*);
 template int engine_run<Pair>(ts_ctx*, EngineJob&, ts_eik_stats*);
 template int engine_run_to_host<double>(ts_ctx*, EngineJob&, void*, int, ts_eik_stats*);
 template int engine_run_to_host<Pair>(ts_ctx*, EngineJob&, void*, int, ts_eik_stats*);

@@ -88,6 +88,11 @@ void engine_field_place(EngineField& f, const FieldLayout& L, int precision, voi
 template <typename Real>
 int engine_run_to_host(ts_ctx* ctx, EngineJob& job, void* out, int out_type, ts_eik_stats* stats);
 
+// One-shot for more fields than the device has room for at once (a row takes a whole number of 32-node tiles there, up
+// to three times its nodes on narrow grids): the fields in runs that fit, each run's results to the host.
+template <typename Real>
+int engine_run_in_parts(ts_ctx* ctx, EngineJob& job, void* out, int out_type, ts_eik_stats* stats);
+
 // Copies padded engine fields to dense grid order (converting to out_type, TS_OUT_F64 / TS_OUT_F32).
 int fields_to_dense_host(ts_ctx* ctx, const EngineJob& job, int precision, void* out, int out_type);
 int fields_to_dense_f32_device(ts_ctx* ctx, const EngineJob& job, int precision, float* out);

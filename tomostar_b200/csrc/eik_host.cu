@@ -253,7 +253,7 @@ static int solve_impl(ts_ctx* ctx, const SolveIn& in, void* out, int out_type, t
     Real* T = nullptr;
     // Many fields into page-locked host memory: the copies of the first half overlap the second half's
     // solve (engine_run_to_host).
-    bool pipelined = false;
+    bool pipelined = false, on_host = false;
     if (in.mode != TS_MODE_PLAIN && out_type != TS_OUT_NONE && out && nf >= 64 && !ctx->use_graph) {
         cudaPointerAttributes at{};
         if (cudaPointerGetAttributes(&at, out) == cudaSuccess) pipelined = at.type == cudaMemoryTypeHost;
@@ -283,6 +283,11 @@ static int solve_impl(ts_ctx* ctx, const SolveIn& in, void* out, int out_type, t
             job.fields.push_back(ef);
         }
         rc = pipelined ? engine_run_to_host<Real>(ctx, job, out, out_type, stats) : engine_run<Real>(ctx, job, stats);
+        on_host = pipelined;
+        if (rc == TS_E_NOMEM && nf > 1 && out_type != TS_OUT_NONE && out) {
+            rc = engine_run_in_parts<Real>(ctx, job, out, out_type, stats);
+            on_host = true;
+        }
         for (auto& ef : job.fields) {
             rounds_max[0] = std::max(rounds_max[0], ef.rounds[0]);
             rounds_max[1] = std::max(rounds_max[1], ef.rounds[1]);
@@ -311,7 +316,7 @@ static int solve_impl(ts_ctx* ctx, const SolveIn& in, void* out, int out_type, t
     const int precision = precision_of<Real>();
     if (out_type == TS_OUT_NONE) return TS_OK;  // the fields stay on the device
     if (in.mode == TS_MODE_PLAIN) return copy_fields_out(ctx, T, precision, int64_t(nf) * n, out, out_type);
-    if (pipelined) return TS_OK;  // already on the host
+    if (on_host) return TS_OK;
     return fields_to_dense_host(ctx, job, precision, out, out_type);
 }
 
