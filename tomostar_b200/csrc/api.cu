@@ -67,19 +67,22 @@ int ts_cuda_create(int32_t device, ts_ctx** out) {
         return TS_E_CUDA;
     }
     {
-        // The context's pool for stream-ordered allocations (without one they come from the device's
+        // The context's pools for stream-ordered allocations (without one they come from the device's
         // default pool, which releases freed memory at every synchronisation).
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        if (cudaMemPoolCreate(&ctx->pool, &props) == cudaSuccess) {
-            uint64_t keep = prop.totalGlobalMem / 4;
-            cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        } else {
-            cudaGetLastError();
-            ctx->pool = nullptr;
-        }
+        auto make = [&](cudaMemPool_t& pool, uint64_t keep) {
+            if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            } else {
+                cudaGetLastError();
+                pool = nullptr;
+            }
+        };
+        make(ctx->pool, prop.totalGlobalMem / 4);
+        make(ctx->table_pool, prop.totalGlobalMem / 32);
     }
     *out = ctx;
     return TS_OK;
@@ -104,8 +107,9 @@ void ts_cuda_destroy(ts_ctx* ctx) {
             if (s) cudaStreamDestroy(s);
         ts::free_copy_slots(ctx);
         cudaStreamDestroy(ctx->stream);
-        // Allocations still held (rows not yet freed) keep the pool's memory until they are freed.
-        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+        // Allocations still held (rows not yet freed) keep a pool's memory until they are freed.
+        for (cudaMemPool_t q : {ctx->pool, ctx->table_pool})
+            if (q) cudaMemPoolDestroy(q);
     }
     delete ctx;
 }

@@ -947,7 +947,7 @@ int ts_tables_upload(ts_ctx* ctx, const ts_grid* grid, int32_t n_tables, const f
     t->n_tables = n_tables;
     t->nodes = int64_t(grid->nx) * grid->ny * grid->nz;
     const size_t bytes = sizeof(float) * size_t(t->nodes) * size_t(n_tables);
-    if (ctx->alloc_async(&t->dev, bytes, ctx->stream) != cudaSuccess) {
+    if (ctx->alloc_tables(&t->dev, bytes) != cudaSuccess) {
         cudaGetLastError();
         delete t;
         return ctx->fail(TS_E_NOMEM, "no device memory for the tables");
@@ -983,7 +983,7 @@ int ts_tables_build(ts_ctx* ctx, const ts_grid* grid, const double* slowness, in
     tb->def = *grid;
     tb->n_tables = n_tables;
     tb->nodes = int64_t(grid->nx) * grid->ny * grid->nz;
-    if (ctx->alloc_async(&tb->dev, sizeof(float) * size_t(tb->nodes) * size_t(n_tables), ctx->stream) != cudaSuccess) {
+    if (ctx->alloc_tables(&tb->dev, sizeof(float) * size_t(tb->nodes) * size_t(n_tables)) != cudaSuccess) {
         cudaGetLastError();
         delete tb;
         return ctx->fail(TS_E_NOMEM, "no device memory for the tables");

@@ -122,7 +122,7 @@ int ts_tables_load_qttb(ts_ctx* ctx, const ts_grid* grid, int32_t count, const c
     t->def = *grid;
     t->n_tables = count;
     t->nodes = n;
-    if (ctx->alloc_async(&t->dev, bytes * size_t(count), ctx->stream) != cudaSuccess) {
+    if (ctx->alloc_tables(&t->dev, bytes * size_t(count)) != cudaSuccess) {
         cudaGetLastError();
         delete t;
         return ctx->fail(TS_E_NOMEM, "no device memory for the tables");
