@@ -1,4 +1,4 @@
-"""Uploads of a context of their own until well past the amount at which they are split over threads (64 MB in all):
+"""Uploads of a context of their own until well past the amount at which they are split over threads (256 MB in all):
 each batch of tables comes back as it went up, from pageable and page-locked memory."""
 import numpy as np
 import pytest
@@ -17,7 +17,7 @@ def test_uploads_add_up(locked):
     g = regular_grid(4, 4, 16, 1.0)  # tables of 1 kB
     rng = np.random.default_rng(1)
     with EikonalCuda.create(0, 64) as e:
-        for kb in (21 * 1024, 2049, 21 * 1024 + 3, 30 * 1024, 21 * 1024 + 1, 3000):
+        for kb in (60 * 1024, 2049, 60 * 1024 + 3, 60 * 1024 + 1, 60 * 1024, 30 * 1024 + 1, 3000):
             tabs = rng.random((kb, g.count), np.float32)
             if locked:
                 tabs = torch.from_numpy(tabs).pin_memory().numpy()

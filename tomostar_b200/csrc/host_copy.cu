@@ -25,10 +25,11 @@ namespace {
 constexpr size_t kSlot = size_t(2) << 20;    // two per thread
 constexpr size_t kSlotBytes = size_t(ts_ctx::kCopyStreams) * 2 * kSlot;
 constexpr size_t kSmall = size_t(2) << 20;   // below this one plain copy is as fast
-// A context's first uploads are plain copies until they add up to this, unless another copy has made the streams:
-// making them and locking the slots takes seven to ten ms once, plain uploads of 64 MB six. From then on a program's
-// uploads gain: 400 rays on 21 MB of tables, call after call, 4.2 ms plain and 3.3 by threads.
-constexpr size_t kFirst = size_t(64) << 20;
+// Until another copy has made the streams, uploads below kFirst are plain copies as long as they have not added up to
+// kAll: making the streams and locking the slots takes seven to ten ms once, a plain upload of 64 MB six, and a
+// server that is given a few models never needs them. From then on a program's uploads gain: 400 rays on 21 MB of
+// tables, call after call, 4.2 ms plain and 3.3 by threads.
+constexpr size_t kFirst = size_t(64) << 20, kAll = 4 * kFirst;
 
 // Runs part(k, slots) for k in [0, n) on n threads (this one among them; a thread that cannot be started
 // leaves its part to this one). The first error of any part.
@@ -95,7 +96,7 @@ int copy_threads(ts_ctx* ctx, const void* host, size_t bytes, bool to_host, char
     cudaGetLastError();
     if (known) return 1;  // page-locked, managed or device memory: the driver's own copy, no host thread may touch it
     if (to_host && bytes < kTouched && touched(host, bytes)) return 1;
-    if (!to_host && !ctx->copy_streams[0] && (ctx->uploaded += bytes) < kFirst) return 1;
+    if (!to_host && !ctx->copy_streams[0] && bytes < kFirst && (ctx->uploaded += bytes) < kAll) return 1;
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
     const int n = int(std::min<size_t>({size_t(ts_ctx::kCopyStreams), size_t(std::max(1u, cores / 2)), bytes / (kSlot / 2)}));
     for (int k = 0; k < n; k++)
